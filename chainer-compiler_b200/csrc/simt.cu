@@ -2,6 +2,8 @@
 // QLinearMatMul, ConvInteger and QLinearConv, plus the small glue kernels of a quantized CNN graph.
 // These are the catch-all path behind the tcgen05 kernels (tc_igemm.cu) and the on-device second
 // opinion the tensor-core results are compared with; they are not the fast path.
+#include <atomic>
+
 #include "common.h"
 #include "epilogue.cuh"
 #include "kernels.h"
@@ -398,96 +400,150 @@ __global__ void __launch_bounds__(256) global_avgpool_dq_kernel(
     y[idx] = __fmul_rn(__fdiv_rn((float)s, (float)HW), scale);
 }
 
-// fp32 Linear: y[n,o] = fma chain over k ascending of x[n,k] * w[o,k], then + b[o].  Every output is accumulated by one
-// thread in k order (no split-K), so the result does not depend on the tiling.  32 x 64 output tile per block of 128
-// threads; a thread owns rows {4 tn .. 4 tn + 3} and columns {to + 16 j}.  A 128-bit shared-memory load costs four cycles
-// of the SM's load unit whatever it broadcasts; the 4 x 4 register tile needs eight of them per 64 fused multiply-adds.  The
-// price of the sequential chains is parallelism: 256 x 1000 outputs are 3.5 warps per SM, about one per scheduler (measured:
-// 63 us for [256, 2048] x [1000, 2048]^T, a quarter of the fp32 rate).  With K-major tiles of pitch 36 floats the loads along k are
-// conflict-free (the eight lanes of a quarter warp read eight different rows whose starts are 36 floats apart, or all the
-// same row).  The next K slice is fetched into registers while the current one is consumed, and shared memory is
-// double-buffered, so there is one barrier per slice.
-constexpr int kLinKS = 32;     // K slice
-constexpr int kLinPitch = 36;  // floats
+// fp32 Linear: y[n,o] = fma chain over k ascending of x[n,k] * w[o,k], then + b[o].  Every output is accumulated by one thread in k order
+// (no split-K), so the result does not depend on the tiling.  The chains leave little parallelism ([256, 2048] x [1000, 2048]^T is 256000
+// chains, one warp per scheduler), so what counts is that a warp never waits: a thread owns an RN x RO register tile, K slices arrive by
+// cp.async several deep, and the shared-memory reads of a later group of four k are issued before the multiply-adds of the current one
+// (with two blocks per SM allowed for, the compiler gave up those registers and a step waited for its loads: 22 us instead of 15 for a
+// single row).
+// Bound: shared-memory reads for many rows (a 128-bit load returns four cycles' worth of bytes whatever it broadcasts; (RN + RO) / (RN RO)
+// of a load per multiply-add, 2x the fp32 pipe's time at 4 x 4), the latency of a chain for few.  Rows are KS + 4 floats apart, so that
+// the eight lanes of a quarter warp read from disjoint banks.
+// Against the single 4 x 4 kernel with one slice in flight: [256, 2048] x [1000, 2048]^T 60.5 -> 45.9 us, [1, 2048] 61.4 -> 14.7 us,
+// [512, 1280] 59.7 -> 49.9 us.
 constexpr int kLinThreads = 128;
 
-__global__ void __launch_bounds__(kLinThreads) linear_f32_kernel(
+// RN x RO: outputs of a thread; TN: threads along n; KS: K slice; STAGES: slices in shared memory; DEPTH: groups of four k in registers.
+template <int RN_, int RO_, int TN_, int KS_, int STAGES_, int DEPTH_>
+struct LinTile {
+    static constexpr int RN = RN_, RO = RO_, TN = TN_, KS = KS_, kStages = STAGES_, kDepth = DEPTH_;
+    static constexpr int TO = kLinThreads / TN;
+    static constexpr int kN = RN * TN, kO = RO * TO, kRows = kN + kO;  // rows of x and of w a block works on
+    static constexpr int kPitch = KS + 4;                               // floats
+    static constexpr int kSmem = kStages * kRows * kPitch * 4;
+};
+
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool valid) {
+    const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
+    const int bytes = valid ? 16 : 0;  // the rest of the sixteen bytes is zero-filled
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(gmem), "r"(bytes) : "memory");
+}
+
+// volatile: keeps the load where it stands, ahead of the multiply-adds it overlaps (the compiler sinks a plain load to its first use)
+__device__ __forceinline__ float4 lds128(uint32_t addr) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
+    return v;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kLinThreads, 1) linear_f32_kernel(
         const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ b, int N, int K, int O, float* __restrict__ y) {
-    __shared__ __align__(16) float Xs[2][32][kLinPitch];
-    __shared__ __align__(16) float Ws[2][64][kLinPitch];
+    constexpr int RN = T::RN, RO = T::RO;
+    extern __shared__ __align__(16) float lin_smem[];  // [stage][kN rows of x, kO rows of w][pitch]
     const int tid = threadIdx.x;
-    const int tn = tid / 16, to = tid % 16;
-    const int n0 = blockIdx.y * 32, o0 = blockIdx.x * 64;
+    const int tn = tid / T::TO, to = tid % T::TO;
+    const int n0 = blockIdx.y * T::kN, o0 = blockIdx.x * T::kO;
     const bool vec = (K % 4 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15u) == 0) && ((reinterpret_cast<uintptr_t>(w) & 15u) == 0);
-    // staging assignment: float4 number f = tid + 128 i of a tile covers row f / 8, k offset 4 (f % 8): two of X, four of W
-    const int sr = tid / 8, sk = (tid % 8) * 4;
-    auto fetch = [&](const float* base, int row, int rows, int k0) -> float4 {
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (row < rows) {
-            const float* p = base + (int64_t)row * K + k0 + sk;
-            if (vec && k0 + sk + 4 <= K) {
-                v = *reinterpret_cast<const float4*>(p);
-            } else {
-                if (k0 + sk + 0 < K) v.x = p[0];
-                if (k0 + sk + 1 < K) v.y = p[1];
-                if (k0 + sk + 2 < K) v.z = p[2];
-                if (k0 + sk + 3 < K) v.w = p[3];
+    const int slices = (K + T::KS - 1) / T::KS;
+    // staging: KS / 4 threads per row, each sixteen bytes of it; rows fr, fr + kStep, ... of the slice
+    constexpr int kPerRow = T::KS / 4, kStep = kLinThreads / kPerRow, kMine = (T::kRows + kStep - 1) / kStep;
+    const int fk = (tid % kPerRow) * 4, fr = tid / kPerRow;
+    const float* src[kMine];
+    bool row_ok[kMine];
+#pragma unroll
+    for (int i = 0; i < kMine; ++i) {
+        const int r = fr + kStep * i;
+        const bool is_x = r < T::kN;
+        const int row = is_x ? n0 + r : o0 + r - T::kN;
+        row_ok[i] = r < T::kRows && row < (is_x ? N : O);
+        src[i] = row_ok[i] ? (is_x ? x : w) + (int64_t)row * K + fk : x;
+    }
+    auto fetch = [&](int sl, int stage) {
+        if (sl < slices) {
+            float* dst = lin_smem + (stage * T::kRows + fr) * T::kPitch + fk;
+            const int k = sl * T::KS + fk;
+#pragma unroll
+            for (int i = 0; i < kMine; ++i) {
+                if (T::kRows % kStep != 0 && fr + kStep * i >= T::kRows) break;
+                if (vec) {
+                    const bool ok = row_ok[i] && k < K;
+                    cp_async16(dst + kStep * i * T::kPitch, ok ? src[i] + sl * T::KS : x, ok);
+                } else {
+                    for (int e = 0; e < 4; ++e) dst[kStep * i * T::kPitch + e] = row_ok[i] && k + e < K ? src[i][sl * T::KS + e] : 0.f;
+                }
             }
         }
-        return v;
+        asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    float acc[4][4] = {};
-    float4 px[2], pw[4];
+    float acc[RN][RO] = {};
 #pragma unroll
-    for (int i = 0; i < 2; ++i) px[i] = fetch(x, n0 + sr + 16 * i, N, 0);
+    for (int i = 0; i < T::kStages - 1; ++i) fetch(i, i);
+    int stage = 0;
+    const uint32_t smem0 = static_cast<uint32_t>(__cvta_generic_to_shared(lin_smem));
+    for (int sl = 0; sl < slices; ++sl) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(T::kStages - 2) : "memory");
+        __syncthreads();  // slice sl has arrived for everyone, and everyone has finished with the buffer that is refilled next
+        fetch(sl + T::kStages - 1, stage == 0 ? T::kStages - 1 : stage - 1);
+        const uint32_t st = smem0 + (uint32_t)(stage * T::kRows * T::kPitch * 4);
+        const uint32_t xs = st + (uint32_t)(tn * RN * T::kPitch * 4), ws = st + (uint32_t)((T::kN + to) * T::kPitch * 4);
+        stage = stage + 1 == T::kStages ? 0 : stage + 1;
+        float4 xv[T::kDepth][RN], wv[T::kDepth][RO];
+        auto load = [&](int buf, int k4) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) pw[i] = fetch(w, o0 + sr + 16 * i, O, 0);
-    int buf = 0;
-    for (int k0 = 0; k0 < K; k0 += kLinKS, buf ^= 1) {
+            for (int i = 0; i < RN; ++i) xv[buf][i] = lds128(xs + (uint32_t)((i * T::kPitch + k4) * 4));
 #pragma unroll
-        for (int i = 0; i < 2; ++i) *reinterpret_cast<float4*>(&Xs[buf][sr + 16 * i][sk]) = px[i];
+            for (int j = 0; j < RO; ++j) wv[buf][j] = lds128(ws + (uint32_t)((j * T::TO * T::kPitch + k4) * 4));
+        };
 #pragma unroll
-        for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(&Ws[buf][sr + 16 * i][sk]) = pw[i];
-        __syncthreads();
-        if (k0 + kLinKS < K) {
-#pragma unroll
-            for (int i = 0; i < 2; ++i) px[i] = fetch(x, n0 + sr + 16 * i, N, k0 + kLinKS);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) pw[i] = fetch(w, o0 + sr + 16 * i, O, k0 + kLinKS);
-        }
+        for (int d = 0; d < T::kDepth - 1; ++d) load(d, d * 4);
         // Elements past K are zero in both operands; fma(0, 0, acc) leaves acc as it is, so the slice is always run in full.
 #pragma unroll
-        for (int k4 = 0; k4 < kLinKS; k4 += 4) {
-            float4 xv[4], wv[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) xv[i] = *reinterpret_cast<const float4*>(&Xs[buf][tn * 4 + i][k4]);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) wv[j] = *reinterpret_cast<const float4*>(&Ws[buf][to + 16 * j][k4]);
-            // k ascending per accumulator; the sixteen accumulators advance together, so that a fused multiply-add never waits
-            // for the one before it (there is only one warp per scheduler to hide that latency)
-            const float xa[4][4] = {{xv[0].x, xv[0].y, xv[0].z, xv[0].w}, {xv[1].x, xv[1].y, xv[1].z, xv[1].w},
-                                    {xv[2].x, xv[2].y, xv[2].z, xv[2].w}, {xv[3].x, xv[3].y, xv[3].z, xv[3].w}};
-            const float wa[4][4] = {{wv[0].x, wv[0].y, wv[0].z, wv[0].w}, {wv[1].x, wv[1].y, wv[1].z, wv[1].w},
-                                    {wv[2].x, wv[2].y, wv[2].z, wv[2].w}, {wv[3].x, wv[3].y, wv[3].z, wv[3].w}};
+        for (int s = 0; s < T::KS / 4; ++s) {
+            if (s + T::kDepth - 1 < T::KS / 4) load((s + T::kDepth - 1) % T::kDepth, (s + T::kDepth - 1) * 4);
+            const float4(&xc)[RN] = xv[s % T::kDepth];
+            const float4(&wc)[RO] = wv[s % T::kDepth];
+            // k ascending per accumulator; the accumulators advance together, so that a multiply-add never waits for the one before it
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk)
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
+                for (int i = 0; i < RN; ++i)
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) acc[i][j] = __fmaf_rn(xa[i][kk], wa[j][kk], acc[i][j]);
+                    for (int j = 0; j < RO; ++j) {
+                        const float xe = kk == 0 ? xc[i].x : (kk == 1 ? xc[i].y : (kk == 2 ? xc[i].z : xc[i].w));
+                        const float we = kk == 0 ? wc[j].x : (kk == 1 ? wc[j].y : (kk == 2 ? wc[j].z : wc[j].w));
+                        acc[i][j] = __fmaf_rn(xe, we, acc[i][j]);
+                    }
         }
-        // the buffer written next iteration is the other one; its readers finished before this iteration's barrier
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int n = n0 + tn * 4 + i;
+    for (int i = 0; i < RN; ++i) {
+        const int n = n0 + tn * RN + i;
         if (n >= N) continue;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int o = o0 + to + 16 * j;
+        for (int j = 0; j < RO; ++j) {
+            const int o = o0 + to + T::TO * j;
             if (o < O) y[(int64_t)n * O + o] = __fadd_rn(acc[i][j], b ? b[o] : 0.f);
         }
     }
+}
+
+template <typename T>
+cudaError_t launch_linear(const float* x, const float* w, const float* b, int N, int K, int O, float* y, cudaStream_t s) {
+    if (T::kSmem > 48 * 1024) {
+        static std::atomic<bool> attr_set[64] = {};  // per device; every writer stores true
+        int dev = 0;
+        const cudaError_t e0 = cudaGetDevice(&dev);
+        if (e0 != cudaSuccess) return e0;
+        if (dev < 0 || dev >= 64 || !attr_set[dev].load(std::memory_order_acquire)) {
+            const cudaError_t e = cudaFuncSetAttribute(linear_f32_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, T::kSmem);
+            if (e != cudaSuccess) return e;
+            if (dev >= 0 && dev < 64) attr_set[dev].store(true, std::memory_order_release);
+        }
+    }
+    const dim3 grid((O + T::kO - 1) / T::kO, (N + T::kN - 1) / T::kN);
+    linear_f32_kernel<T><<<grid, kLinThreads, T::kSmem, s>>>(x, w, b, N, K, O, y);
+    return cudaGetLastError();
 }
 
 // NCHW <-> NHWC transposes through a 32x32 shared tile over the (C, H*W) plane.
@@ -728,8 +784,17 @@ extern "C" int chxq_global_avgpool_dq_nhwc(const uint8_t* x, int32_t N, int32_t 
 
 extern "C" int chxq_linear_f32(const float* x, const float* w, const float* b, int32_t N, int32_t K, int32_t O, float* y, void* stream) {
     CHXQ_CHECK_ARG(x && w && y && N > 0 && K > 0 && O > 0, "Linear: bad arguments");
-    dim3 grid((O + 63) / 64, (N + 31) / 32);
-    linear_f32_kernel<<<grid, kLinThreads, 0, as_stream(stream)>>>(x, w, b, N, K, O, y);
+    // The largest register tile that still puts a block on every second SM (4 x 4: 2048 outputs per block; measured at K = 2048, O = 1000:
+    // 192 rows 46 us as 4 x 4 and 48 as 2 x 2, 128 rows 44 and 38); for a few tens of rows the single-output tile, whose chains are
+    // the shortest.
+    const int64_t outputs = (int64_t)N * O;
+    cudaStream_t s = as_stream(stream);
+    if (outputs >= (int64_t)80 * 2048)
+        CHXQ_CUDA((launch_linear<LinTile<4, 4, 8, 64, 4, 2>>(x, w, b, N, K, O, y, s)));
+    else if (outputs >= 40000)
+        CHXQ_CUDA((launch_linear<LinTile<2, 2, 8, 64, 5, 3>>(x, w, b, N, K, O, y, s)));
+    else
+        CHXQ_CUDA((launch_linear<LinTile<1, 1, 4, 128, 5, 5>>(x, w, b, N, K, O, y, s)));
     CHXQ_LAUNCH_CHECK();
     return CHXQ_OK;
 }

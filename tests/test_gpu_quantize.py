@@ -192,3 +192,13 @@ def test_prepare_weights_matches_host_quantizer_and_merge(pkg, ops, orc, dev, to
     from chainer_compiler_b200 import _lib
     with pytest.raises(_lib.ChxqError):
         ops.PrepareWeights(torch.zeros((4, 3), device=dev), (torch.ones(3, device=dev),) * 4)
+
+
+@pytest.mark.parametrize("n,k,o", [(1, 1, 1), (5, 130, 33), (3, 127, 1000), (41, 1280, 1000), (40, 68, 1001), (164, 66, 1000), (170, 2048, 1003)])
+def test_linear_tiles(ops, orc, dev, n, k, o):
+    """Every register tile of the fp32 Linear at ragged extents (rows, columns and K slices that do not fill a tile, K with and without
+    16-byte rows): the k-ascending chain of the oracle, bit for bit."""
+    rng = np.random.default_rng(n * 7 + k)
+    x, w = rng.standard_normal((n, k)).astype(np.float32), rng.standard_normal((o, k)).astype(np.float32)
+    b = rng.standard_normal(o).astype(np.float32)
+    assert np.array_equal(ops.Linear(_t(x, dev), _t(w, dev), _t(b, dev)).cpu().numpy(), orc.linear_f32(x, w, b))
