@@ -125,6 +125,29 @@ static int largest_pow2_divisor(int v, int cap) {
     return d;
 }
 
+// The position tile: 128 output positions as a box of Wb x Hb x Nb (powers of two).  Powers of two that divide the map waste nothing when
+// the batch fills the box, but on maps with odd extents they leave everything to the image axis (1 x 1 x 128 on a 7 x 7 map), and a batch
+// smaller than that computes padding: one image of 14 x 14 ran as 49 tiles of four positions.  So the box with the fewest tiles is taken;
+// the dividing one where it is not beaten.  Loads beyond the map are zero fill, stores are clipped.
+static void choose_tile(const chxq_conv_geom& g, TcConvPlan* pl) {
+    auto tiles = [&](int wb, int hb, int nb) {
+        return (int64_t)((g.Wo + wb - 1) / wb) * ((g.Ho + hb - 1) / hb) * ((g.N + nb - 1) / nb);
+    };
+    pl->Wb = largest_pow2_divisor(g.Wo, 16);
+    pl->Hb = largest_pow2_divisor(g.Ho, 128 / pl->Wb);
+    pl->Nb = 128 / (pl->Wb * pl->Hb);
+    int64_t best = tiles(pl->Wb, pl->Hb, pl->Nb);
+    for (int wb = 16; wb >= 1; wb /= 2)
+        for (int hb = 128 / wb; hb >= 1; hb /= 2) {
+            if (hb * g.stride_h > 256) continue;  // extent of a TMA box
+            const int64_t t = tiles(wb, hb, 128 / (wb * hb));
+            if (t < best) {
+                best = t;
+                pl->Wb = wb; pl->Hb = hb; pl->Nb = 128 / (wb * hb);
+            }
+        }
+}
+
 TcConvPlan plan_tc_conv(const chxq_conv_geom& g) {
     TcConvPlan pl{};
     pl.path = kTcNone;
@@ -149,9 +172,7 @@ TcConvPlan plan_tc_conv(const chxq_conv_geom& g) {
         pl.c_pitch = depthwise ? 64 : (cg + pl.bk - 1) / pl.bk * pl.bk;
         pl.k_total = taps * pl.c_pitch;
         pl.a_pitch = pl.k_total;
-        pl.Wb = largest_pow2_divisor(g.Wo, 16);
-        pl.Hb = largest_pow2_divisor(g.Ho, 128 / pl.Wb);
-        pl.Nb = 128 / (pl.Wb * pl.Hb);
+        choose_tile(g, &pl);
         return pl;
     }
     // Stride-2 convolutions over at most 4 channels (network stems): space-to-depth.  A 2x2 pixel block becomes one
@@ -170,9 +191,7 @@ TcConvPlan plan_tc_conv(const chxq_conv_geom& g) {
             pl.kh2 = kh2; pl.kw2 = kw2; pl.t0h = t0h; pl.t0w = t0w;
             pl.rows2 = g.Ho + kh2 - 1;
             pl.cols2 = g.Wo + pl.bk / 16 - 1;  // the last window of a row ends inside the row, zero weights beyond kw2 blocks
-            pl.Wb = largest_pow2_divisor(g.Wo, 16);
-            pl.Hb = largest_pow2_divisor(g.Ho, 128 / pl.Wb);
-            pl.Nb = 128 / (pl.Wb * pl.Hb);
+            choose_tile(g, &pl);
             return pl;
         }
     }
@@ -190,9 +209,7 @@ TcConvPlan plan_tc_conv(const chxq_conv_geom& g) {
             // 1x1: the map is a plain [N*H*W, C] matrix.
             pl.Wb = 128; pl.Hb = 1; pl.Nb = 1;
         } else {
-            pl.Wb = largest_pow2_divisor(g.Wo, 16);
-            pl.Hb = largest_pow2_divisor(g.Ho, 128 / pl.Wb);
-            pl.Nb = 128 / (pl.Wb * pl.Hb);
+            choose_tile(g, &pl);
         }
         return pl;
     }
