@@ -1,6 +1,7 @@
 // C-ABI entry points of the contraction ops (MatMulInteger, QLinearMatMul, ConvInteger, QLinearConv):
 // argument validation, convolution geometry, path selection, workspace carving, and the small
 // pre-pass kernels that feed the tensor-core kernel (operand repacking and zero-point terms).
+#include <cooperative_groups.h>
 #include <string.h>
 
 #include <atomic>
@@ -28,10 +29,6 @@ __device__ __forceinline__ int zp_at(const ZpSpec& z, int64_t i, int is_signed) 
     return ldq_rt(z.ptr, z.len == 1 ? 0 : i, is_signed);
 }
 
-// B[K, N] (row-major) -> Bt[N, k_pad] (K-major rows, zero padded) and, in the same pass, the column terms of the activation zero
-// point, T[n] += sum_k za[k] * b[k, n] (T zeroed beforehand; integer atomics, so the sum is exact whatever the order).
-// 64 x 64 bytes per block of 256 threads: 32-bit loads along N, a 4 x 4 byte transpose in registers, the tile through shared
-// memory as words with a pitch of 17 (conflict-free), 128-bit stores along K.
 __device__ __forceinline__ void transpose4x4(uint32_t (&r)[4]) {
     const uint32_t t0 = __byte_perm(r[0], r[1], 0x5140), t1 = __byte_perm(r[0], r[1], 0x7362);
     const uint32_t t2 = __byte_perm(r[2], r[3], 0x5140), t3 = __byte_perm(r[2], r[3], 0x7362);
@@ -41,78 +38,129 @@ __device__ __forceinline__ void transpose4x4(uint32_t (&r)[4]) {
     r[3] = __byte_perm(t1, t3, 0x7632);
 }
 
-__global__ void __launch_bounds__(256) transpose_b_terms_kernel(
+// Four bytes at any address, of which the first n (1 .. 4, more reads as 4) belong to the buffer.  The words that hold them are read
+// aligned, and only those that hold at least one of them: no access leaves the four-byte words of the buffer.
+__device__ __forceinline__ uint32_t load4_unaligned(const uint8_t* p, int64_t n) {
+    const uintptr_t addr = reinterpret_cast<uintptr_t>(p);
+    const int mis = (int)(addr & 3u);
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(addr - (uintptr_t)mis);
+    const uint32_t lo = __ldg(w);
+    const uint32_t hi = (mis != 0 && n > 4 - mis) ? __ldg(w + 1) : 0u;
+    const uint32_t v = __funnelshift_r(lo, hi, 8 * mis);
+    return n >= 4 ? v : v & ((1u << (8 * (int)n)) - 1u);
+}
+
+// B[K, N] (row-major) -> Bt[N, k_pad] (K-major rows, zero padded) and, in the same pass, the column terms of the activation zero
+// point, T[n] = sum_k za[k] * b[k, n], and the widened column zero points zbn[n] (either may be absent).
+// Bound: memory (B read once, written once).  A cluster of eight blocks owns 64 columns and takes their 64-row tiles in turn, so that the
+// sums stay in the cluster: they meet in the first block through distributed shared memory, where single-tile blocks needed a memset
+// launch in front and global atomics.  A tile: 32-bit loads along N at any alignment of the rows, a 4 x 4 byte transpose in registers, the
+// tile through shared memory as words with a pitch of 17 (conflict-free), 128-bit stores along K.
+constexpr int kTrSplit = 8;
+__global__ void __cluster_dims__(1, kTrSplit, 1) __launch_bounds__(256) transpose_b_terms_kernel(
         const uint8_t* __restrict__ b, int64_t K, int64_t N, int64_t k_pad, uint8_t* __restrict__ bt, ZpSpec za, int a_signed, int b_signed,
-        int32_t* __restrict__ T) {
-    __shared__ uint32_t tw[64][17];
+        int32_t* __restrict__ T, ZpSpec zb, int32_t* __restrict__ zbn) {
+    __shared__ uint32_t tw[2][64][17];
     __shared__ int colsum[64];
     const int tid = threadIdx.x;
-    const int64_t k0 = (int64_t)blockIdx.y * 64, n0 = (int64_t)blockIdx.x * 64;
-    const int a = tid / 16, bq = tid % 16;  // load side: rows k0 + 4a .. +3, columns n0 + 4bq .. +3
+    const int64_t n0 = (int64_t)blockIdx.x * 64;
+    const int a = tid / 16, bq = tid % 16;   // load side: rows k0 + 4a .. +3, columns n0 + 4bq .. +3
+    const int col = tid / 4, q = tid % 4;    // store side: column n0 + col, rows k0 + 16q .. +15
     const bool words_ok = (N % 4 == 0) && ((reinterpret_cast<uintptr_t>(b) & 3u) == 0);
     if (tid < 64) colsum[tid] = 0;
-    uint32_t r[4];
+    const int64_t k_tiles = (k_pad + 63) / 64;
+    const int64_t n = n0 + 4 * bq;
     int part[4] = {0, 0, 0, 0};
+    auto load = [&](int64_t kt, uint32_t (&r)[4]) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int64_t k = k0 + 4 * a + i, n = n0 + 4 * bq;
-        uint32_t v = 0u;
-        if (k < K && n < N) {
-            const uint8_t* src = b + k * N + n;
-            if (words_ok && n + 4 <= N) {
-                v = *reinterpret_cast<const uint32_t*>(src);
-            } else {
-                for (int j = 0; j < 4 && n + j < N; ++j) v |= (uint32_t)src[j] << (8 * j);
+        for (int i = 0; i < 4; ++i) {
+            const int64_t k = kt * 64 + 4 * a + i;
+            uint32_t v = 0u;
+            if (kt < k_tiles && k < K && n < N) {
+                const uint8_t* src = b + k * N + n;
+                v = words_ok ? __ldg(reinterpret_cast<const uint32_t*>(src)) : load4_unaligned(src, N - n);
             }
-            if (T != nullptr) {
-                const int z = zp_at(za, k, a_signed);
+            r[i] = v;
+        }
+    };
+    uint32_t r[4];
+    load(blockIdx.y, r);
+    int buf = 0;
+    for (int64_t kt = blockIdx.y; kt < k_tiles; kt += kTrSplit, buf ^= 1) {
+        uint32_t next[4];
+        load(kt + kTrSplit, next);
+        if (T != nullptr) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int64_t k = kt * 64 + 4 * a + i;
+                const int z = k < K ? zp_at(za, k, a_signed) : 0;
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    const uint32_t byte = (v >> (8 * j)) & 0xffu;
+                    const uint32_t byte = (r[i] >> (8 * j)) & 0xffu;
                     part[j] += z * (b_signed ? (int)(int8_t)byte : (int)byte);
                 }
             }
         }
-        r[i] = v;
-    }
-    transpose4x4(r);  // r[j] = rows 4a .. 4a+3 of column 4bq + j
-    __syncthreads();   // colsum is zero
+        transpose4x4(r);  // r[j] = rows 4a .. 4a+3 of column 4bq + j
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        tw[4 * bq + j][a] = r[j];
-        if (T != nullptr && part[j] != 0) atomicAdd(&colsum[4 * bq + j], part[j]);
-    }
-    __syncthreads();
-    const int col = tid / 4, q = tid % 4;  // store side: column n0 + col, rows k0 + 16q .. +15
-    const int64_t n = n0 + col, k = k0 + 16 * q;
-    if (n < N && k < k_pad) {
-        const uint32_t w4[4] = {tw[col][4 * q], tw[col][4 * q + 1], tw[col][4 * q + 2], tw[col][4 * q + 3]};
-        uint8_t* dst = bt + n * k_pad + k;
-        if (k + 16 <= k_pad && ((reinterpret_cast<uintptr_t>(dst) & 15u) == 0)) {
-            *reinterpret_cast<uint4*>(dst) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
-        } else {
-            for (int j = 0; j < 16 && k + j < k_pad; ++j) dst[j] = (uint8_t)(w4[j >> 2] >> (8 * (j & 3)));
+        for (int j = 0; j < 4; ++j) tw[buf][4 * bq + j][a] = r[j];
+        __syncthreads();  // the other buffer's readers finished before they came here
+        const int64_t k = kt * 64 + 16 * q;
+        if (n0 + col < N && k < k_pad) {  // k_pad is a multiple of 64: whole 16-byte pieces, aligned (bt is)
+            const uint32_t* w4 = &tw[buf][col][4 * q];
+            *reinterpret_cast<uint4*>(bt + (n0 + col) * k_pad + k) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
         }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) r[i] = next[i];
     }
-    if (T != nullptr && tid < 64 && n0 + tid < N && colsum[tid] != 0) atomicAdd(&T[n0 + tid], colsum[tid]);
+    if (T != nullptr) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            part[j] += __shfl_xor_sync(0xffffffffu, part[j], 16);  // the warp's two row groups
+            if ((tid & 16) == 0 && part[j] != 0) atomicAdd(&colsum[4 * bq + j], part[j]);
+        }
+        cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+        cluster.sync();
+        if (cluster.block_rank() == 0 && tid < 64 && n0 + tid < N) {
+            int s = 0;
+#pragma unroll
+            for (int i = 0; i < kTrSplit; ++i) s += cluster.map_shared_rank(colsum, i)[tid];
+            T[n0 + tid] = s;
+        }
+        cluster.sync();  // a block's shared memory stays until it has been read
+    }
+    if (zbn != nullptr && blockIdx.y == 0 && tid < 64 && n0 + tid < N) zbn[n0 + tid] = zp_at(zb, n0 + tid, b_signed);
 }
 
-// zbn[n] = zb[n] widened.  One thread per column.
-__global__ void __launch_bounds__(256) gemm_zb_kernel(int b_signed, int64_t N, ZpSpec zb, int32_t* __restrict__ zbn) {
-    const int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (n < N) zbn[n] = zp_at(zb, n, b_signed);
-}
-
-// R[m] = sum_k (a[m, k] - za[k]).  One warp per row.
-__global__ void __launch_bounds__(256) gemm_row_terms_kernel(const void* __restrict__ a, int a_signed, int64_t M, int64_t K, ZpSpec za, int32_t* __restrict__ R) {
+// One warp per row of A: R[m] = sum_k (a[m, k] - za[k]) (absent: null), and the row at a pitch TMA can describe (K rounded up to sixteen
+// bytes, zero padded; absent: null).  Sixteen bytes per lane, read as aligned words at whatever address the row starts.
+__global__ void __launch_bounds__(256) gemm_a_rows_kernel(
+        const uint8_t* __restrict__ a, int a_signed, int64_t M, int64_t K, ZpSpec za, int64_t pitch, uint8_t* __restrict__ out, int32_t* __restrict__ R) {
     const int64_t m = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (m >= M) return;
+    const uint8_t* row = a + m * K;
+    const bool aligned = (reinterpret_cast<uintptr_t>(row) & 15u) == 0;
     int s = 0;
-    for (int64_t k = lane; k < K; k += 32) s += ldq_rt(a, m * K + k, a_signed) - zp_at(za, k, a_signed);
+    for (int64_t k = 16 * lane; k < K; k += 16 * 32) {
+        uint32_t w[4];
+        if (aligned && k + 16 <= K) {
+            const uint4 v = __ldg(reinterpret_cast<const uint4*>(row + k));
+            w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) w[i] = k + 4 * i < K ? load4_unaligned(row + k + 4 * i, K - k - 4 * i) : 0u;
+        }
+        if (out != nullptr) *reinterpret_cast<uint4*>(out + m * pitch + k) = make_uint4(w[0], w[1], w[2], w[3]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) s = a_signed ? __dp4a((int)w[i], 0x01010101, s) : (int)__dp4a(w[i], 0x01010101u, (unsigned)s);
+        if (R != nullptr && za.len > 1)
+            for (int i = 0; i < 16 && k + i < K; ++i) s -= zp_at(za, k + i, a_signed);
+    }
+    if (R == nullptr) return;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) R[m] = s;
+    if (lane == 0) R[m] = za.len == 1 ? s - (int)K * zp_at(za, 0, a_signed) : s;
 }
 
 // OIHW weights -> K-major rows [M][tap * c_pitch + c], zero padded to k_total.  One thread per output byte.
@@ -386,9 +434,10 @@ inline int blocks_for(int64_t threads_needed, int block = 256) {
 // GEMM dispatch shared by MatMulInteger and QLinearMatMul.
 // ---------------------------------------------------------------------------------------------
 struct GemmWs {
-    size_t bt_off, t_off, zbn_off, r_off, total;
+    size_t bt_off, t_off, zbn_off, r_off, a_off, total;
     int bk;
     int64_t k_pad;
+    int64_t a_pitch;  // bytes between rows of A as the kernel reads them: K, or, where that is no multiple of sixteen, of the copy at a_off
 };
 
 GemmWs gemm_ws_layout(int64_t M, int64_t N, int64_t K) {
@@ -400,6 +449,9 @@ GemmWs gemm_ws_layout(int64_t M, int64_t N, int64_t K) {
     w.t_off = off; off += align_up((size_t)N * 4, 256);
     w.zbn_off = off; off += align_up((size_t)N * 4, 256);
     w.r_off = off; off += align_up((size_t)M * 4, 256);
+    w.a_off = off;
+    w.a_pitch = (K + 15) / 16 * 16;
+    if (w.a_pitch != K) off += align_up((size_t)M * (size_t)w.a_pitch, 256);
     w.total = off;
     return w;
 }
@@ -409,13 +461,20 @@ bool gemm_tc_eligible(const void* a, int64_t M, int64_t N, int64_t K) {
            K < (1ll << 31);
 }
 
+// Rows of A that do not start on sixteen-byte boundaries (K % 16 != 0) reach the tensor cores through a copy at a wider pitch.  The copy
+// is one pass over A; the CUDA-core kernel makes one multiply-add per lane and clock.  One B200, whole calls: 509 x 3073 x 1283 with zero
+// points 293 -> 41 us, the 784-1000-1000-10 MLP of 64 rows (two of its three products have K = 1000) 103.5 -> 66 us.
+bool gemm_tc_via_copy(int64_t M, int64_t N, int64_t K) {
+    return K % 16 != 0 && K >= 16 && M >= 1 && N >= 1 && M < (1ll << 31) && N < (1ll << 31) && K < (1ll << 20);
+}
+
 int gemm_dispatch(
         const char* op, const void* a, bool a_signed, const void* b, bool b_signed, int64_t batch, int64_t M, int64_t N, int64_t K,
         const ZpSpec& za, const ZpSpec& zb, const EpiArgs& epi, void* y, size_t y_elem, void* workspace, size_t workspace_bytes, int path,
         cudaStream_t s) {
     if (batch == 0 || M == 0 || N == 0) return CHXQ_OK;
     const bool tc_ok = gemm_tc_eligible(a, M, N, K) && ((M * K) % 16 == 0 || batch == 1);
-    bool use_tc = path == CHXQ_PATH_TENSOR || (path == CHXQ_PATH_AUTO && tc_ok);
+    bool use_tc = path == CHXQ_PATH_TENSOR || (path == CHXQ_PATH_AUTO && (tc_ok || gemm_tc_via_copy(M, N, K)));
     if (path == CHXQ_PATH_TENSOR && !tc_ok)
         return set_error(CHXQ_ERR_UNSUPPORTED, "%s: tensor-core path needs K %% 16 == 0 and a 16-byte aligned A (M=%lld N=%lld K=%lld)", op,
                          (long long)M, (long long)N, (long long)K);
@@ -433,34 +492,33 @@ int gemm_dispatch(
     const GemmWs ws = gemm_ws_layout(M, N, K);
     uint8_t* wsp = static_cast<uint8_t*>(workspace);
     uint8_t* bt = wsp + ws.bt_off;
-    int32_t* T = reinterpret_cast<int32_t*>(wsp + ws.t_off);
-    int32_t* zbn = reinterpret_cast<int32_t*>(wsp + ws.zbn_off);
-    int32_t* R = reinterpret_cast<int32_t*>(wsp + ws.r_off);
+    int32_t* T = za.len > 0 ? reinterpret_cast<int32_t*>(wsp + ws.t_off) : nullptr;
+    int32_t* zbn = zb.len > 0 ? reinterpret_cast<int32_t*>(wsp + ws.zbn_off) : nullptr;
+    int32_t* R = zb.len > 0 ? reinterpret_cast<int32_t*>(wsp + ws.r_off) : nullptr;
+    uint8_t* a_copy = ws.a_pitch != K ? wsp + ws.a_off : nullptr;
     for (int64_t bi = 0; bi < batch; ++bi) {
         const uint8_t* ab = static_cast<const uint8_t*>(a) + bi * M * K;
         const uint8_t* bb = static_cast<const uint8_t*>(b) + bi * K * N;
-        dim3 tgrid((unsigned)((N + 63) / 64), (unsigned)((ws.k_pad + 63) / 64));
-        if (tgrid.y > 65535) return set_error(CHXQ_ERR_UNSUPPORTED, "%s: K too large for the repacking grid", op);
-        // one pass over B: the K-major copy and, when a has a zero point, its column terms
-        if (za.len > 0) CHXQ_CUDA(cudaMemsetAsync(T, 0, (size_t)N * 4, s));
-        transpose_b_terms_kernel<<<tgrid, 256, 0, s>>>(bb, K, N, ws.k_pad, bt, za, a_signed ? 1 : 0, b_signed ? 1 : 0, za.len > 0 ? T : nullptr);
-        if (zb.len > 0) {
-            gemm_zb_kernel<<<blocks_for(N), 256, 0, s>>>(b_signed ? 1 : 0, N, zb, zbn);
-            gemm_row_terms_kernel<<<blocks_for(M * 32), 256, 0, s>>>(ab, a_signed, M, K, za, R);
-            count_launch(2);
+        if ((ws.k_pad + 63) / 64 > 65535) return set_error(CHXQ_ERR_UNSUPPORTED, "%s: K too large for the tensor-core path", op);
+        if (a_copy != nullptr || R != nullptr) {
+            gemm_a_rows_kernel<<<blocks_for(M * 32), 256, 0, s>>>(ab, a_signed ? 1 : 0, M, K, za, ws.a_pitch, a_copy, R);
+            CHXQ_LAUNCH_CHECK();
         }
+        // one pass over B: the K-major copy, the column terms of a's zero point and b's zero points widened
+        transpose_b_terms_kernel<<<dim3((unsigned)((N + 63) / 64), kTrSplit), 256, 0, s>>>(bb, K, N, ws.k_pad, bt, za, a_signed ? 1 : 0,
+                                                                                           b_signed ? 1 : 0, T, zb, zbn);
         CHXQ_LAUNCH_CHECK();
         TcProblem p{};
-        p.a = ab; p.a_signed = a_signed; p.C = (int)K; p.a_cs = K; p.W = (int)M; p.H = 1; p.N = 1;
+        p.a = a_copy ? a_copy : ab; p.a_signed = a_signed; p.C = (int)K; p.a_cs = ws.a_pitch; p.W = (int)M; p.H = 1; p.N = 1;
         p.b = bt; p.b_signed = b_signed; p.cols = (int)N; p.c_pad = (int)ws.k_pad; p.bk = ws.bk;
         p.KH = 1; p.KW = 1; p.pad_top = 0; p.pad_left = 0;
         p.Wo = (int)M; p.Ho = 1; p.No = 1; p.Wb = 128; p.Hb = 1; p.Nb = 1; p.bn = 0;
         p.y = static_cast<uint8_t*>(y) + (size_t)bi * M * N * y_elem;
         p.ldc = N;
-        p.col_corr = za.len > 0 ? T : nullptr;
+        p.col_corr = T;
         p.col_scale = 1;
-        p.col_mul = zb.len > 0 ? zbn : nullptr;
-        p.row_corr = zb.len > 0 ? R : nullptr;
+        p.col_mul = zbn;
+        p.row_corr = R;
         p.epi = epi;
         p.alg_macs = (double)M * (double)N * (double)K;
         if (epi.residual) p.epi.residual = epi.residual + (size_t)bi * M * N;

@@ -283,6 +283,17 @@ void* scratch(size_t nbytes, const at::Tensor& like) {
     return nbytes == 0 ? nullptr : scratch_tensor(nbytes, like.device()).data_ptr();
 }
 
+// Scratch of one call, from the caching allocator on the call's stream: calls on several streams or threads stay independent of one another.
+// (The shared buffer orders nothing between streams.)
+struct OwnScratch {
+    at::Tensor t;
+    void* get(size_t nbytes, const at::Tensor& like) {
+        if (nbytes == 0) return nullptr;
+        t = at::detail::empty_cuda({(int64_t)nbytes}, at::kByte, like.device(), std::nullopt);
+        return t.data_ptr();
+    }
+};
+
 // ---- QLinearConv parameters -----------------------------------------------------------------------------------------------
 
 // Whether a weight zero-point tensor holds only zeros, learned by ONE device-to-host read per tensor (and again after an in-place change,
@@ -575,7 +586,8 @@ PyObject* matmul_integer(PyObject*, Args a, Py_ssize_t n) {
     const int path = (int)as_long(a[4]);
     at::Tensor y = empty_map(size, at::kInt, l, false);
     const size_t ws_bytes = path != CHXQ_PATH_SIMT ? chxq_matmul_integer_workspace(batch, M, N, K) : 0;
-    void* ws = scratch(ws_bytes, l);
+    OwnScratch own;
+    void* ws = K % 16 != 0 ? own.get(ws_bytes, l) : scratch(ws_bytes, l);
     call([&] {
         return chxq_matmul_integer(l.data_ptr(), cl, r.data_ptr(), cr, batch, M, N, K, za.ptr, za.len, zb.ptr, zb.len, static_cast<int32_t*>(y.data_ptr()), ws,
                                    ws_bytes, path, stream());
@@ -601,7 +613,8 @@ PyObject* qlinear_matmul(PyObject*, Args a, Py_ssize_t n) {
     const int mode = (int)as_long(a[8]), path = (int)as_long(a[9]);
     at::Tensor y = empty_map({M, N}, qtype(zy.code), l, false);
     const size_t ws_bytes = path != CHXQ_PATH_SIMT ? chxq_matmul_integer_workspace(1, M, N, K) : 0;
-    void* ws = scratch(ws_bytes, l);
+    OwnScratch own;
+    void* ws = K % 16 != 0 ? own.get(ws_bytes, l) : scratch(ws_bytes, l);
     call([&] {
         return chxq_qlinear_matmul(l.data_ptr(), cl, sa, za.value, r.data_ptr(), cr, sb, zb.value, sy, zy.value, zy.code, M, N, K, mode, y.data_ptr(), ws,
                                    ws_bytes, path, stream());
