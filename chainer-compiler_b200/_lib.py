@@ -121,6 +121,8 @@ SIGNATURES = {
     "chxq_dynamic_quant_params_u8": (_c.c_int, [_vp, _vp, _vp, _vp, _vp]),
     "chxq_quantize_linear_dev": (_c.c_int, [_vp, _i64, _vp, _vp, _i32, _i32, _vp, _vp]),
     "chxq_conv_integer_dev": (_c.c_int, [_vp, _vp, _vp, _vp, _vp, _i64, _vp, _vp]),
+    "chxq_conv_dev_workspace": (_sz, [_c.POINTER(ConvGeom)]),
+    "chxq_conv_integer_dev_ws": (_c.c_int, [_vp, _vp, _vp, _vp, _vp, _i64, _vp, _vp, _sz, _vp]),
 }
 
 _lib = None

@@ -163,6 +163,188 @@ __global__ void __launch_bounds__(256) gemm_a_rows_kernel(
     if (lane == 0) R[m] = za.len == 1 ? s - (int)K * zp_at(za, 0, a_signed) : s;
 }
 
+// Everything a convolution over NCHW maps (or with a device-resident zero point) needs in front of the tensor-core kernel, as one launch.
+// Blocks [0, M): one output channel each -- its weights from OIHW to the K-major row [tap * c_pitch + c] (zero padded), their sum times the
+// activation zero point, and its own zero point widened.  The other blocks: 128 positions of the input map each, transposed to NHWC rows of
+// cs channels (zero padded), with a border of the activation zero point around the map where the convolution pads (`border`; the reference
+// pads after subtracting the zero point, and TMA's zero fill can only express a zero point of 0), and per pixel the sum of (x - zx) over the
+// block's share of the channels, from which the GEMM's epilogue gathers the weight zero-point term of a window.
+// Bound: one read and one write of the map.  Transpose and packing were four launches with a byte-wise path for maps whose extent is no
+// multiple of four; a padded map with a zero point went through an im2col matrix, KH * KW times the bytes, and a map with a device zero
+// point through the one-thread-per-output CUDA-core kernel.  One B200: the dynamically quantized
+// 3 x 3 convolution of [8, 64, 56, 56], four operators, 1186 -> 45 us; the pass itself 13.6 us for 25.7 MB in and out.
+struct ConvPrep {
+    const uint8_t* x;
+    const uint8_t* w;
+    const void* x_zp_dev;  // device zero point, else x_zp
+    int x_zp, x_signed, w_signed;
+    int N, C, H, W, M, taps;
+    int x_nhwc;
+    int64_t x_cs;               // NHWC input: channel stride
+    int border, pt, pl, Hp, Wp;  // extents of the map written
+    int cs;                     // its channel stride (multiple of 16)
+    int pos_tiles, parts, tiles_per_part;  // 128-position tiles per image, channel shares of ceil(tiles) 64-channel tiles
+    int c_pitch, k_total;
+    ZpSpec zw;
+    uint8_t* x_out;
+    int32_t* pix;  // [parts][N][Hp * Wp], or null
+    uint8_t* w_out;
+    int32_t* wsum_zx;
+    int32_t* zw32;
+};
+
+// kNhwc: the input is NHWC; kBorder: a border is written; kPix: pixel sums.
+constexpr int kPrepPos = 128, kPrepPitch = 132;  // positions of a tile; words between channel quads (16-byte aligned, two-way conflicts at most)
+template <bool kNhwc, bool kBorder, bool kPix>
+__global__ void __launch_bounds__(256) conv_prep_kernel(const ConvPrep a) {
+    __shared__ __align__(16) uint32_t tw[16 * kPrepPitch];  // [channel quad][position]: four channels of a position per word
+    __shared__ int warp_sum[8];
+    const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+    const int zx = a.x_zp_dev ? ldq_rt(a.x_zp_dev, 0, a.x_signed) : a.x_zp;
+    if ((int)blockIdx.x < a.M) {
+        const int m = blockIdx.x;
+        const uint8_t* row = a.w + (int64_t)m * a.C * a.taps;
+        uint32_t* dst = reinterpret_cast<uint32_t*>(a.w_out + (int64_t)m * a.k_total);
+        int s = 0;
+        for (int i = tid; i < a.k_total / 4; i += 256) {
+            const int tap = 4 * i / a.c_pitch, c = 4 * i - tap * a.c_pitch;
+            uint32_t v = 0u;
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (tap < a.taps && c + j < a.C) v |= (uint32_t)row[(int64_t)(c + j) * a.taps + tap] << (8 * j);
+            dst[i] = v;
+            s = a.w_signed ? __dp4a((int)v, 0x01010101, s) : (int)__dp4a(v, 0x01010101u, (unsigned)s);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) warp_sum[warp] = s;
+        __syncthreads();
+        if (tid == 0) {
+#pragma unroll
+            for (int i = 1; i < 8; ++i) s += warp_sum[i];
+            a.wsum_zx[m] = (int)((unsigned)s * (unsigned)zx);
+            a.zw32[m] = zp_at(a.zw, m, a.w_signed);
+        }
+        return;
+    }
+    unsigned b = blockIdx.x - (unsigned)a.M;
+    const int part = (int)(b % (unsigned)a.parts);
+    b /= (unsigned)a.parts;
+    const int p0 = (int)(b % (unsigned)a.pos_tiles) * kPrepPos;
+    const int n = (int)(b / (unsigned)a.pos_tiles);
+    const int plane = a.Hp * a.Wp, HW = a.H * a.W;
+    // load side (NCHW): this lane's four positions of the written map, for channel quads `warp` and `warp + 8` of a 64-channel tile
+    const int lp = p0 + 4 * lane;
+    int lh = 0, lw = 0;
+    bool run = lp < plane;  // four consecutive input bytes (the last ones of a map without border may be fewer)
+    if (kBorder && !kNhwc) {
+        lh = lp / a.Wp - a.pt;
+        lw = lp % a.Wp - a.pl;
+        run = run && lh >= 0 && lh < a.H && lw >= 0 && lw + 4 <= a.W;
+    }
+    const int run_off = kBorder ? lh * a.W + lw : lp;
+    const bool words = !kBorder && HW % 4 == 0 && (reinterpret_cast<uintptr_t>(a.x) & 3u) == 0;
+    // store side: positions p0 + tid / 4 and 64 further, channels 16q .. +15
+    const int q = tid % 4;
+    int sum[2] = {0, 0}, real = 0;
+    const int c_first = part * a.tiles_per_part * 64, c_end = min(a.cs, c_first + a.tiles_per_part * 64);
+    for (int c0 = c_first; c0 < c_end; c0 += 64) {
+        if (!kNhwc) {
+            uint32_t r[2][4];
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int ch = c0 + 4 * (warp + 8 * h) + i;
+                    uint32_t v = 0u;
+                    if (ch < a.C && lp < plane) {
+                        const uint8_t* src = a.x + ((int64_t)n * a.C + ch) * HW;
+                        if (words) {
+                            v = __ldg(reinterpret_cast<const uint32_t*>(src + lp));
+                        } else if (run) {
+                            v = load4_unaligned(src + run_off, kBorder ? 4 : HW - lp);
+                        } else {
+                            int y = lh, x = lw;
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                const bool in = y >= 0 && y < a.H && x >= 0 && x < a.W;
+                                if (lp + j < plane) v |= (in ? (uint32_t)src[(int64_t)y * a.W + x] : (uint32_t)zx & 0xffu) << (8 * j);
+                                if (++x + a.pl == a.Wp) {
+                                    x = -a.pl;
+                                    ++y;
+                                }
+                            }
+                        }
+                    }
+                    r[h][i] = v;
+                }
+            if (c0 != c_first) __syncthreads();  // the previous channel tile has been read
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                transpose4x4(r[h]);  // r[h][j] = the quad's channels of position lp + j
+                *reinterpret_cast<uint4*>(tw + (warp + 8 * h) * kPrepPitch + 4 * lane) = make_uint4(r[h][0], r[h][1], r[h][2], r[h][3]);
+            }
+            __syncthreads();
+        }
+        const int c = c0 + 16 * q;
+        const int in_c = max(0, min(16, a.C - c));
+        real += in_c;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int pos = tid / 4 + 64 * h, sp = p0 + pos;
+            if (sp >= plane || c >= a.cs) continue;
+            uint32_t w4[4] = {0u, 0u, 0u, 0u};
+            if (!kNhwc) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) w4[i] = tw[(4 * q + i) * kPrepPitch + pos];
+            } else {
+                const int y = sp / a.Wp - a.pt, x = sp % a.Wp - a.pl;
+                const bool in = !kBorder || (y >= 0 && y < a.H && x >= 0 && x < a.W);
+                const uint8_t* src = a.x + (((int64_t)n * a.H + y) * a.W + x) * a.x_cs + c;
+                if (in && in_c == 16 && (reinterpret_cast<uintptr_t>(src) & 15u) == 0) {
+                    const uint4 v = __ldg(reinterpret_cast<const uint4*>(src));
+                    w4[0] = v.x; w4[1] = v.y; w4[2] = v.z; w4[3] = v.w;
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                        if (j < in_c) w4[j / 4] |= (in ? (uint32_t)src[j] : (uint32_t)zx & 0xffu) << (8 * (j % 4));
+                }
+            }
+            *reinterpret_cast<uint4*>(a.x_out + ((int64_t)n * plane + sp) * a.cs + c) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
+            if (kPix) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) sum[h] = a.x_signed ? __dp4a((int)w4[i], 0x01010101, sum[h]) : (int)__dp4a(w4[i], 0x01010101u, (unsigned)sum[h]);
+            }
+        }
+    }
+    if (kPix) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            int s = sum[h] - real * zx;
+            s += __shfl_xor_sync(0xffffffffu, s, 1);
+            s += __shfl_xor_sync(0xffffffffu, s, 2);
+            const int sp = p0 + tid / 4 + 64 * h;
+            if (q == 0 && sp < plane) a.pix[((int64_t)part * a.N + n) * plane + sp] = s;
+        }
+    }
+}
+
+int launch_conv_prep(const ConvPrep& a, cudaStream_t s) {
+    const unsigned grid = (unsigned)((int64_t)a.pos_tiles * a.N * a.parts + a.M);
+    switch ((a.x_nhwc ? 4 : 0) + (a.border ? 2 : 0) + (a.pix ? 1 : 0)) {
+        case 0: conv_prep_kernel<false, false, false><<<grid, 256, 0, s>>>(a); break;
+        case 1: conv_prep_kernel<false, false, true><<<grid, 256, 0, s>>>(a); break;
+        case 2: conv_prep_kernel<false, true, false><<<grid, 256, 0, s>>>(a); break;
+        case 3: conv_prep_kernel<false, true, true><<<grid, 256, 0, s>>>(a); break;
+        case 4: conv_prep_kernel<true, false, false><<<grid, 256, 0, s>>>(a); break;
+        case 5: conv_prep_kernel<true, false, true><<<grid, 256, 0, s>>>(a); break;
+        case 6: conv_prep_kernel<true, true, false><<<grid, 256, 0, s>>>(a); break;
+        default: conv_prep_kernel<true, true, true><<<grid, 256, 0, s>>>(a); break;
+    }
+    CHXQ_LAUNCH_CHECK();
+    return CHXQ_OK;
+}
+
 // OIHW weights -> K-major rows [M][tap * c_pitch + c], zero padded to k_total.  One thread per output byte.
 __global__ void __launch_bounds__(256) pack_weights_kernel(
         const uint8_t* __restrict__ w, int M, int C, int taps, int c_pitch, int k_total, uint8_t* __restrict__ out) {
@@ -759,6 +941,132 @@ bool nchw_plan(const chxq_conv_geom& g, size_t y_elem, NchwPlan* out) {
     return true;
 }
 
+// The one-launch form of the above for dense convolutions: conv_prep_kernel in front, the tensor-core kernel on the map it wrote.  Also runs
+// convolutions whose activation zero point is on the device.
+struct PrepPlan {
+    chxq_conv_geom g;  // the NHWC problem on the written map
+    TcConvPlan pl;
+    ConvPrep prep;     // everything but the pointers
+    size_t blob_off, x_off, pix_off, y_off, total;
+};
+
+bool prep_plan(const chxq_conv_geom& g, int y_elem, bool border, bool pixel_sums, PrepPlan* out) {
+    if (g.group != 1 || g.stride_h > 8 || g.stride_w > 8 || g.pad_top < 0 || g.pad_left < 0 || g.pad_bottom < 0 || g.pad_right < 0) return false;
+    const bool padded = g.pad_top || g.pad_left || g.pad_bottom || g.pad_right;
+    border = padded && (border || g.pad_top >= g.KH || g.pad_left >= g.KW);
+    const int64_t Hp = g.H + (border ? g.pad_top + g.pad_bottom : 0), Wp = g.W + (border ? g.pad_left + g.pad_right : 0);
+    const int taps = g.KH * g.KW;
+    PrepPlan& P = *out;
+    P = PrepPlan{};
+    P.g = g;
+    P.g.x_layout = CHXQ_NHWC;
+    P.g.H = (int)Hp; P.g.W = (int)Wp;
+    if (border) P.g.pad_top = P.g.pad_left = P.g.pad_bottom = P.g.pad_right = 0;
+    ConvPrep& a = P.prep;
+    a.cs = (g.C + 15) / 16 * 16;
+    P.g.x_cstride = a.cs;
+    const bool y_nchw = g.y_layout == CHXQ_NCHW;
+    if (y_nchw) {
+        P.g.y_layout = CHXQ_NHWC;
+        P.g.y_cstride = (g.M + 15) / 16 * 16;
+    }
+    const int64_t rows = (int64_t)g.N * g.Ho * g.Wo;
+    P.pl = plan_tc_conv_direct(P.g);
+    if (Hp * Wp >= (1 << 30) || (int64_t)g.H * g.W >= (1 << 30) || (int64_t)g.M * P.pl.k_total >= (1ll << 31) || rows >= (1ll << 31)) return false;
+    a.N = g.N; a.C = g.C; a.H = g.H; a.W = g.W; a.M = g.M; a.taps = taps;
+    a.x_nhwc = g.x_layout == CHXQ_NHWC;
+    a.x_cs = a.x_nhwc ? (g.x_cstride > 0 ? g.x_cstride : g.C) : 0;
+    a.x_signed = g.x_dtype == CHXQ_INT8; a.w_signed = g.w_dtype == CHXQ_INT8;
+    a.border = border; a.pt = border ? g.pad_top : 0; a.pl = border ? g.pad_left : 0;
+    a.Hp = (int)Hp; a.Wp = (int)Wp;
+    a.c_pitch = P.pl.c_pitch; a.k_total = P.pl.k_total;
+    a.pos_tiles = (int)((Hp * Wp + kPrepPos - 1) / kPrepPos);
+    // Channel tiles side by side where nothing is summed over them; with pixel sums a block keeps its channels, in up to four shares
+    // (each is another load per tap in the epilogue) where the positions alone leave SMs idle.
+    const int c_tiles = (a.cs + 63) / 64;
+    int parts = c_tiles;
+    if (pixel_sums) {
+        const int64_t blocks = (int64_t)a.pos_tiles * g.N;
+        parts = (int)(blocks >= 592 ? 1 : (592 + blocks - 1) / (blocks > 0 ? blocks : 1));
+        if (parts > 4) parts = 4;
+        if (parts > c_tiles) parts = c_tiles;
+    }
+    a.tiles_per_part = (c_tiles + parts - 1) / parts;
+    a.parts = (c_tiles + a.tiles_per_part - 1) / a.tiles_per_part;
+    if ((int64_t)a.pos_tiles * g.N * a.parts + g.M >= (1ll << 31)) return false;
+    const ConvWs L = conv_ws_layout(P.g, P.pl);
+    size_t off = 0;
+    P.blob_off = off; off += L.pack_total;
+    off = align_up(off, 1024);
+    P.x_off = off; off += align_up((size_t)g.N * (size_t)(Hp * Wp) * a.cs, 1024);
+    P.pix_off = off;
+    if (pixel_sums) off += align_up((size_t)a.parts * g.N * (size_t)(Hp * Wp) * 4, 1024);
+    P.y_off = off;
+    if (y_nchw && y_elem == 1) off += align_up((size_t)rows * P.g.y_cstride, 1024);
+    P.total = off;
+    return true;
+}
+
+size_t prep_workspace(const chxq_conv_geom& g) {  // the largest over the forms a call may take
+    PrepPlan P;
+    return prep_plan(g, 1, true, true, &P) ? P.total : 0;
+}
+
+int conv_prep_run(const void* x, const void* w, const chxq_conv_geom& g, PrepPlan& P, int x_zp, const void* x_zp_dev, const ZpSpec& zw,
+                  const EpiArgs& epi, void* y, uint8_t* wsp, cudaStream_t s) {
+    const ConvWs L = conv_ws_layout(P.g, P.pl);
+    uint8_t* blob = wsp + P.blob_off;
+    ConvPrep& a = P.prep;
+    a.x = static_cast<const uint8_t*>(x); a.w = static_cast<const uint8_t*>(w);
+    a.x_zp_dev = x_zp_dev; a.x_zp = x_zp; a.zw = zw;
+    a.x_out = wsp + P.x_off;
+    a.pix = zw.len > 0 ? reinterpret_cast<int32_t*>(wsp + P.pix_off) : nullptr;
+    a.w_out = blob + L.pack_off;
+    a.wsum_zx = reinterpret_cast<int32_t*>(blob + L.wsum_off);
+    a.zw32 = reinterpret_cast<int32_t*>(blob + L.zw_off);
+    const int prep_rc = launch_conv_prep(a, s);
+    if (prep_rc != CHXQ_OK) return prep_rc;
+    const int64_t rows = (int64_t)g.N * g.Ho * g.Wo;
+    TcProblem p{};
+    p.a = a.x_out; p.C = a.cs; p.a_cs = a.cs;
+    const bool flat = P.pl.Wb == 128;  // a 1x1 convolution over the flattened map
+    if (flat) {
+        p.W = (int)rows; p.H = 1; p.N = 1;
+        p.Wo = (int)rows; p.Ho = 1; p.No = 1;
+    } else {
+        p.W = P.g.W; p.H = P.g.H; p.N = g.N;
+        p.Wo = g.Wo; p.Ho = g.Ho; p.No = g.N;
+    }
+    p.c_pad = P.pl.c_pitch; p.KH = g.KH; p.KW = g.KW; p.pad_top = P.g.pad_top; p.pad_left = P.g.pad_left;
+    p.sw = g.stride_w; p.sh = g.stride_h;
+    p.Wb = P.pl.Wb; p.Hb = P.pl.Hb; p.Nb = P.pl.Nb;
+    p.a_signed = a.x_signed;
+    p.b = a.w_out; p.b_signed = a.w_signed; p.cols = g.M; p.bk = P.pl.bk;
+    p.col_corr = x_zp_dev != nullptr || x_zp != 0 ? a.wsum_zx : nullptr;
+    p.col_scale = 1;
+    if (zw.len > 0) {
+        p.col_mul = a.zw32;
+        p.row_corr = a.pix;
+        p.win_w = flat ? (int)rows : P.g.W; p.win_h = flat ? 1 : P.g.H; p.win_parts = a.parts;
+    }
+    p.epi = epi;
+    p.alg_macs = (double)rows * g.M * g.C * a.taps;
+    const bool y_nchw = g.y_layout == CHXQ_NCHW;
+    if (!y_nchw) {
+        p.y = y; p.ldc = g.y_cstride > 0 ? g.y_cstride : g.M;
+        return launch_tc_igemm(p, s);
+    }
+    p.ldc = P.g.y_cstride;
+    if (epi.mode == kEpiInt32) {
+        p.y = y;
+        p.y_plane = (int64_t)g.Ho * g.Wo;
+        return launch_tc_igemm(p, s);
+    }
+    p.y = wsp + P.y_off;
+    const int rc = launch_tc_igemm(p, s);
+    return rc != CHXQ_OK ? rc : chxq_nhwc_to_nchw(p.y, 1, g.N, g.M, g.Ho, g.Wo, P.g.y_cstride, y, s);
+}
+
 size_t inner_conv_workspace(const chxq_conv_geom& g2) {
     const TcConvPlan pl = plan_tc_conv(g2);
     if (pl.path == kTcNone) return 0;
@@ -784,7 +1092,22 @@ int conv_dispatch(
     }
     if (path == CHXQ_PATH_AUTO && g->group > 1 && epi.mode == kEpiRequant && depthwise_eligible(*g, x, y, epi.residual))
         return launch_depthwise(x, w, *g, xz, zw.ptr, zw.len, epi, y, s);
-    // NCHW in, NCHW out (the reference's signature): NHWC inside, transposes around it, when the caller's workspace has room.
+    // NCHW in, NCHW out (the reference's signature): NHWC inside, when the caller's workspace has room.
+    PrepPlan pp;
+    if (path != CHXQ_PATH_SIMT && epi.residual == nullptr && g->C > 4 && g->x_layout == CHXQ_NCHW && g->y_layout == CHXQ_NCHW && g->N <= 65535 &&
+        prep_plan(*g, epi.mode == kEpiInt32 ? 4 : 1, xz != 0, zw.len != 0, &pp)) {
+        if (workspace != nullptr && workspace_bytes >= pp.total && (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0) {
+            rc = conv_prep_run(x, w, *g, pp, xz, nullptr, zw, epi, y, static_cast<uint8_t*>(workspace), s);
+            if (!(rc == CHXQ_ERR_UNSUPPORTED && path == CHXQ_PATH_AUTO)) return rc;
+            return launch_conv_simt(x, w, *g, has_x_zp, x_zp, zw.ptr, zw.len, epi, y, s);
+        }
+        if (path == CHXQ_PATH_TENSOR)
+            return set_error(CHXQ_ERR_WORKSPACE, "%s: the tensor-core path behind NCHW tensors needs %zu bytes of 256-byte aligned workspace (got %zu)", op,
+                             pp.total, workspace_bytes);
+        return launch_conv_simt(x, w, *g, has_x_zp, x_zp, zw.ptr, zw.len, epi, y, s);
+    }
+    // what that form does not take (maps of at most four channels, which the stem paths read as NCHW themselves; groups): transposes
+    // around the NHWC call
     NchwPlan np;
     if (path != CHXQ_PATH_SIMT && epi.residual == nullptr && nchw_plan(*g, epi.mode == kEpiInt32 ? 4 : 1, &np)) {
         const size_t need = np.x_bytes + np.y_bytes + inner_conv_workspace(np.g2);
@@ -1062,6 +1385,8 @@ extern "C" int chxq_conv_resolve_geometry(
 
 extern "C" size_t chxq_conv_workspace(const chxq_conv_geom* g) {
     if (!g || validate_geom("conv workspace", g) != CHXQ_OK) return 0;
+    PrepPlan pp;
+    if (g->C > 4 && g->x_layout == CHXQ_NCHW && g->y_layout == CHXQ_NCHW && g->N <= 65535 && prep_plan(*g, 1, true, true, &pp)) return pp.total;
     NchwPlan np;
     if (nchw_plan(*g, 4, &np)) return np.x_bytes + np.y_bytes + inner_conv_workspace(np.g2);  // sized for int32 outputs (ConvInteger), the larger case
     const TcConvPlan pl = plan_tc_conv(*g);
@@ -1107,6 +1432,26 @@ extern "C" int chxq_conv_integer_dev(
     EpiArgs epi{};
     epi.mode = kEpiInt32;
     return launch_conv_simt(x, w, *g, 1, 0, w_zero_point, w_zp_len, epi, y, as_stream(stream), x_zero_point);
+}
+
+extern "C" size_t chxq_conv_dev_workspace(const chxq_conv_geom* g) {
+    if (!g || validate_geom("conv workspace", g) != CHXQ_OK) return 0;
+    return prep_workspace(*g);
+}
+
+extern "C" int chxq_conv_integer_dev_ws(
+        const void* x, const void* w, const chxq_conv_geom* g, const void* x_zero_point, const void* w_zero_point, int64_t w_zp_len, int32_t* y,
+        void* workspace, size_t workspace_bytes, void* stream) {
+    PrepPlan pp;
+    if (g != nullptr && validate_geom("ConvInteger", g) == CHXQ_OK && (int64_t)g->N * g->M * g->Ho * g->Wo != 0 && x && w && y && x_zero_point &&
+        check_zp_len("ConvInteger", "w_zero_point", w_zero_point, w_zp_len, g->M) == CHXQ_OK && prep_plan(*g, 4, true, w_zp_len != 0, &pp) &&
+        workspace != nullptr && workspace_bytes >= pp.total && (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0) {
+        EpiArgs epi{};
+        epi.mode = kEpiInt32;
+        const int rc = conv_prep_run(x, w, *g, pp, 0, x_zero_point, ZpSpec{w_zero_point, w_zp_len, 0}, epi, y, static_cast<uint8_t*>(workspace), as_stream(stream));
+        if (rc != CHXQ_ERR_UNSUPPORTED) return rc;
+    }
+    return chxq_conv_integer_dev(x, w, g, x_zero_point, w_zero_point, w_zp_len, y, stream);  // the general kernel, and its errors
 }
 
 extern "C" int chxq_qlinear_conv(

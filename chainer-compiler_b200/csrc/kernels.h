@@ -82,6 +82,10 @@ struct TcProblem {
     int col_scale;
     const int32_t* col_mul;
     const int32_t* row_corr;
+    // win_w > 0: row_corr is not indexed by position but holds per-pixel sums over the input channels, [win_parts][N][win_h][win_w] (one
+    // part per share of the channels); a position's term is their sum over its KH x KW window, pixels outside counting zero.
+    int win_w, win_h, win_parts;
+    int64_t y_plane;  // > 0 (int32 outputs only): y is [image][cols][y_plane], y_plane = output positions per image; ldc is not used
     EpiArgs epi;
     double alg_macs;  // multiply-accumulates of the problem as the op defines it (no padding), for profiling
     // Fused 3x3 / stride-2 / pad-0 max pooling of the uint8 output: y is then the pooled map [No, pool_ho, pool_wo] x ldc and the
@@ -111,6 +115,7 @@ struct TcConvPlan {
     int group_cols, group_cin, diag;
 };
 TcConvPlan plan_tc_conv(const chxq_conv_geom& g);
+TcConvPlan plan_tc_conv_direct(const chxq_conv_geom& g);  // the direct plan of a dense NHWC geometry whose channel stride is a multiple of 16
 int choose_bk(int k);
 
 }  // namespace chxq

@@ -639,7 +639,10 @@ PyObject* conv_integer(PyObject*, Args a, Py_ssize_t n) {
         const at::Tensor& zx = THPVariable_Unpack(a[2]);
         if (zx.scalar_type() != x.scalar_type()) fail(CHXQ_ERR_INVALID_ARGUMENT, "ConvInteger: a device x_zero_point must have x's dtype");
         const ZpArray zw = zp_array(a[3], w, "w_zero_point");
-        call([&] { return chxq_conv_integer_dev(x.data_ptr(), w.data_ptr(), &g, zx.data_ptr(), zw.ptr, zw.len, yp, stream()); });
+        OwnScratch own;
+        const size_t ws_bytes = chxq_conv_dev_workspace(&g);
+        void* ws = own.get(ws_bytes, x);
+        call([&] { return chxq_conv_integer_dev_ws(x.data_ptr(), w.data_ptr(), &g, zx.data_ptr(), zw.ptr, zw.len, yp, ws, ws_bytes, stream()); });
         return wrap(std::move(y));
     }
     const Zp zx = zp_scalar(a[2]);

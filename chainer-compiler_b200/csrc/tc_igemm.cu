@@ -148,6 +148,23 @@ static void choose_tile(const chxq_conv_geom& g, TcConvPlan* pl) {
         }
 }
 
+TcConvPlan plan_tc_conv_direct(const chxq_conv_geom& g) {
+    TcConvPlan pl{};
+    pl.path = kTcDirect;
+    pl.bk = choose_bk(g.C);
+    pl.c_pitch = (g.C + pl.bk - 1) / pl.bk * pl.bk;
+    pl.k_total = g.KH * g.KW * pl.c_pitch;
+    pl.a_pitch = pl.k_total;
+    if (g.KH * g.KW == 1 && g.stride_h == 1 && g.stride_w == 1 && g.pad_top == 0 && g.pad_left == 0 && g.pad_bottom == 0 && g.pad_right == 0 &&
+        (int64_t)g.N * g.H * g.W < (1ll << 31)) {
+        // 1x1: the map is a plain [N*H*W, C] matrix.
+        pl.Wb = 128; pl.Hb = 1; pl.Nb = 1;
+    } else {
+        choose_tile(g, &pl);
+    }
+    return pl;
+}
+
 TcConvPlan plan_tc_conv(const chxq_conv_geom& g) {
     TcConvPlan pl{};
     pl.path = kTcNone;
@@ -198,21 +215,7 @@ TcConvPlan plan_tc_conv(const chxq_conv_geom& g) {
     const bool direct = g.x_layout == CHXQ_NHWC && g.stride_h >= 1 && g.stride_w >= 1 && g.stride_h <= 8 && g.stride_w <= 8 && (xcs % 16 == 0) &&
                         g.pad_top >= 0 && g.pad_left >= 0 &&
                         g.pad_bottom >= 0 && g.pad_right >= 0 && g.pad_top < g.KH && g.pad_left < g.KW && g.C >= 16;
-    if (direct) {
-        pl.path = kTcDirect;
-        pl.bk = choose_bk(g.C);
-        pl.c_pitch = (g.C + pl.bk - 1) / pl.bk * pl.bk;
-        pl.k_total = taps * pl.c_pitch;
-        pl.a_pitch = pl.k_total;
-        if (taps == 1 && g.stride_h == 1 && g.stride_w == 1 && g.pad_top == 0 && g.pad_left == 0 && g.pad_bottom == 0 && g.pad_right == 0 &&
-            (int64_t)g.N * g.H * g.W < (1ll << 31)) {
-            // 1x1: the map is a plain [N*H*W, C] matrix.
-            pl.Wb = 128; pl.Hb = 1; pl.Nb = 1;
-        } else {
-            choose_tile(g, &pl);
-        }
-        return pl;
-    }
+    if (direct) return plan_tc_conv_direct(g);
     // Everything else with one group: explicit im2col into workspace, then a plain GEMM.
     // NCHW maps with up to 4 channels (a network stem) use one 32-bit word per pixel: channel pitch 4.
     const int cp = (g.x_layout == CHXQ_NCHW && g.C < 4) ? 4 : g.C;
@@ -271,6 +274,9 @@ int launch_tc_igemm(const TcProblem& q, cudaStream_t s) {
     // 10-12 (0 = u8, 1 = s8), both operands K-major (bits 15, 16 = 0), N >> 3 in bits 17-22, M >> 4 in bits 24-28.
     p.idesc = (2u << 4) | ((q.a_signed ? 1u : 0u) << 7) | ((q.b_signed ? 1u : 0u) << 10) | ((uint32_t)(bn >> 3) << 17) | ((128u >> 4) << 24);
     p.col_corr = q.col_corr; p.col_scale = q.col_scale; p.col_mul = q.col_mul; p.row_corr = q.row_corr;
+    p.win_w = q.win_w; p.win_h = q.win_h; p.win_parts = q.win_parts;
+    p.y_plane = q.y_plane;
+    if (p.y_plane > 0 && epi_kind != tc::kEpiKInt32) return set_error(CHXQ_ERR_UNSUPPORTED, "tensor-core kernel: NCHW stores are for int32 outputs");
     p.epi = q.epi;
     p.y = q.y;
 #ifdef CHXQ_TL

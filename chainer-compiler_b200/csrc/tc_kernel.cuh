@@ -242,6 +242,36 @@ __device__ __forceinline__ void umma_i8_lohi(uint32_t tmem_d, uint32_t a_lo, uin
             : "memory");
 }
 
+// Weight zero-point term of an output position: the sum of (x - zx) over its receptive field, stored per position or gathered from per-pixel
+// sums (a 3 x 3 window is nine cached loads per position and tile, where a pass of its own would cost a launch).
+__device__ __forceinline__ uint32_t row_term(const TcParams& p, int no, int ho, int wo, int64_t pos) {
+    if (p.row_corr == nullptr) return 0u;
+    if (p.win_w == 0) return (uint32_t)p.row_corr[pos];
+    uint32_t s = 0u;
+    for (int part = 0; part < p.win_parts; ++part) {
+        const int32_t* img = p.row_corr + ((int64_t)part * p.No + no) * p.win_h * p.win_w;
+        for (int kh = 0; kh < p.KH; ++kh) {
+            const int h = ho * p.sh - p.pad_top + kh;
+            if (h < 0 || h >= p.win_h) continue;
+            for (int kw = 0; kw < p.KW; ++kw) {
+                const int w = wo * p.sw - p.pad_left + kw;
+                if (w >= 0 && w < p.win_w) s += (uint32_t)__ldg(img + (int64_t)h * p.win_w + w);
+            }
+        }
+    }
+    return s;
+}
+
+// Stores n of the sixteen int32 outputs of a position as NCHW: neighbouring lanes own neighbouring positions of an image row, so a store of
+// one channel covers whole 32-byte sectors without a transposing pass.
+__device__ __forceinline__ void store_nchw16(const TcParams& p, int64_t pos, int cbase, int n, const uint32_t (&r)[16]) {
+    const int64_t img = pos / p.y_plane;
+    int32_t* yo = static_cast<int32_t*>(p.y) + (img * p.cols + cbase) * p.y_plane + (pos - img * p.y_plane);
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+        if (j < n) yo[j * p.y_plane] = (int32_t)r[j];
+}
+
 template <int BN, int BK>
 struct TcConfig {
     static constexpr int kStageA = 128 * BK;
@@ -450,6 +480,8 @@ tc_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             };
             uint4 res0 = res_load(0), res1 = res_load(1);
 
+            uint32_t rowc = 0u;
+            if ((EPI == kEpiKInt32 || EPI == kEpiKGeneric) && p.col_mul && row_ok) rowc = row_term(p, no, ho, wo, pos);
             const bool got = mbar_wait(tfull_bar(acc), acc_phase, abort_flag, p.status, 4, 32, p.wait_limit_ns);
             if (!__all_sync(0xffffffffu, got)) break;
             tc_fence_after();
@@ -481,7 +513,6 @@ tc_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 }
                 if (EPI == kEpiKInt32 || EPI == kEpiKGeneric) {
                     if (p.col_mul) {  // weight zero-point term: - zw[c] * sum over the receptive field of (x - zx)
-                        const uint32_t rowc = p.row_corr ? (uint32_t)p.row_corr[pos] : 0u;
 #pragma unroll
                         for (int j = 0; j < 16; ++j)
                             if (full_chunk || cbase + j < p.cols) r[j] -= (uint32_t)__ldg(p.col_mul + cbase + j) * rowc;
@@ -489,7 +520,9 @@ tc_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 }
                 if (EPI == kEpiKInt32) {
                     int32_t* yo = static_cast<int32_t*>(p.y) + o;
-                    if (full_chunk && p.vec_ok) {
+                    if (p.y_plane > 0) {
+                        store_nchw16(p, pos, cbase, p.cols - cbase, r);
+                    } else if (full_chunk && p.vec_ok) {
 #pragma unroll
                         for (int j = 0; j < 4; ++j)
                             reinterpret_cast<uint4*>(yo)[j] = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);

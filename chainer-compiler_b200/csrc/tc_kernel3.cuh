@@ -399,7 +399,7 @@ tc_igemm3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 const int wo = w0 + w_l, ho = h0 + h_l, no = n0 + n_l;
                 const bool row_ok = pt < pos_tiles && wo < p.Wo && ho < p.Ho && no < p.No;
                 const int64_t pos = ((int64_t)no * p.Ho + ho) * p.Wo + wo;
-                const uint32_t rowc = (p.row_corr && row_ok) ? (uint32_t)p.row_corr[pos] : 0u;  // sum over the row of (a - za), for the weight zero points
+                const uint32_t rowc = (p.col_mul && row_ok) ? row_term(p, no, ho, wo, pos) : 0u;  // sum over the row of (a - za), for the weight zero points
                 const bool got = mbar_wait(tfull_bar(acc), acc_phase, abort_flag, p.status, 4, 32);
                 if (!__all_sync(0xffffffffu, got)) break;
                 tc_fence_after();
@@ -421,7 +421,9 @@ tc_igemm3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                     }
                     if (!row_ok) continue;
                     int32_t* yo = static_cast<int32_t*>(p.y) + pos * p.ldc + cbase;
-                    if (p.vec_ok && cbase + 16 <= p.cols) {
+                    if (p.y_plane > 0) {
+                        store_nchw16(p, pos, cbase, p.cols - cbase, r);
+                    } else if (p.vec_ok && cbase + 16 <= p.cols) {
 #pragma unroll
                         for (int j = 0; j < 4; ++j) reinterpret_cast<uint4*>(yo)[j] = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
                     } else {

@@ -34,6 +34,8 @@ struct TcParams {
     int col_scale;
     const int32_t* col_mul;
     const int32_t* row_corr;
+    int win_w, win_h, win_parts;  // row_corr as pixel sums (TcProblem::win_w); win_w == 0: one value per position
+    int64_t y_plane;              // int32 outputs: positions per image of an NCHW output, 0 = rows of ldc elements
     EpiArgs epi;
     void* y;
     int* status;

@@ -358,14 +358,18 @@ int chxq_minmax_f32(const float* x, int64_t n, float* out2, void* stream);
  *   chxq_quantize_linear_dev: chxq_quantize_linear with y_scale and y_zero_point (dtype y_dtype, may be NULL = 0) read from
  *     device memory; same element arithmetic (runtime/ops/quantize.cc:16-35).
  *   chxq_conv_integer_dev: chxq_conv_integer (runtime/ops/quantize.cc:116-146) with the activation zero point read from a device
- *     scalar of x's dtype; runs on the general CUDA-core kernel (the tensor-core path folds a host-known zero point into its
- *     padding value and correction terms).
+ *     scalar of x's dtype; without scratch it runs on the general CUDA-core kernel.
+ *   chxq_conv_integer_dev_ws: the same on the tensor cores, with chxq_conv_dev_workspace bytes of 256-byte aligned scratch; falls back to
+ *     the general kernel where the geometry has no such form (groups, negative pads, strides above 8) or the scratch is too small.
  * MatMulInteger already takes its zero points as device arrays. */
 int chxq_dynamic_quant_params_u8(const float* rmin, const float* rmax, float* scale, uint8_t* zero_point, void* stream);
 int chxq_quantize_linear_dev(const float* x, int64_t n, const float* y_scale, const void* y_zero_point, int32_t y_dtype, int32_t round_mode,
                              void* y, void* stream);
 int chxq_conv_integer_dev(const void* x, const void* w, const chxq_conv_geom* g, const void* x_zero_point, const void* w_zero_point,
                           int64_t w_zp_len, int32_t* y, void* stream);
+size_t chxq_conv_dev_workspace(const chxq_conv_geom* g);
+int chxq_conv_integer_dev_ws(const void* x, const void* w, const chxq_conv_geom* g, const void* x_zero_point, const void* w_zero_point,
+                             int64_t w_zp_len, int32_t* y, void* workspace, size_t workspace_bytes, void* stream);
 
 #ifdef __cplusplus
 }
