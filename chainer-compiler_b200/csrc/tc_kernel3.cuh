@@ -197,6 +197,19 @@ tc_igemm3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     const int taps = p.KH * p.KW;
     const int num_kb = taps * p.c_chunks;
 
+    // Which 256-channel block and which pair of position tiles an item is.  Eight column blocks at a time, all position pairs of those before
+    // the next eight: the 74 pairs at work then share about nine blocks of A and eight of B, 36 MB of K = 8192 operands where whole rows of a
+    // wide product were 2.3 blocks of A and all of B, past what one die's half of the L2 holds.  QLinearMatMul 8192^3 on one B200: 491 -> 475 us.
+    constexpr int kGroupCols = 8;
+    auto item_coords = [&](int item, int& ct, int& pair) {
+        const int per_group = p.col_tiles <= kGroupCols ? 0 : kGroupCols * pos_pairs;
+        const int g = p.col_tiles <= kGroupCols ? 0 : item / per_group;
+        const int width = min(kGroupCols, p.col_tiles - g * kGroupCols);
+        const int within = item - g * per_group;
+        pair = within / width;
+        ct = g * kGroupCols + within - pair * width;
+    };
+
     // Output coordinates of position tile `pt` (a tile past the end lands beyond the last image: loads fill zero, its store is skipped).
     auto tile_origin = [&](int pt, int& w0, int& h0, int& n0) {
         const int tw = pt % p.tiles_w;
@@ -223,8 +236,9 @@ tc_igemm3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             const int tlmax = is_a ? 512 : 256;
 #endif
             for (int item = first_item; item < total_items && ok; item += num_pairs_launched, ++it) {
-                const int ct = item % p.col_tiles;
-                const int pt = (item / p.col_tiles) * 2 + (int)rank;
+                int ct, pair;
+                item_coords(item, ct, pair);
+                const int pt = pair * 2 + (int)rank;
                 int w0, h0, n0;
                 tile_origin(pt, w0, h0, n0);
                 if (RES && is_a) {
@@ -354,7 +368,8 @@ tc_igemm3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         for (int item = first_item; item < total_items; item += num_pairs_launched, ++it) {
             const int acc = it & 1;
             const uint32_t acc_phase = (uint32_t)(it >> 1) & 1u;
-            const int ct = item % p.col_tiles;
+            int ct, pair;
+            item_coords(item, ct, pair);
             const int col0 = ct * BN;
             const int buf = it % kBufsDiv;
 
@@ -392,7 +407,7 @@ tc_igemm3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             if constexpr (kInt32) {
                 // int32 outputs: every thread owns one output position (row) and writes its sixteen accumulators of a chunk as 64
                 // contiguous bytes, straight from registers.
-                const int pt = (item / p.col_tiles) * 2 + (int)rank;
+                const int pt = pair * 2 + (int)rank;
                 int w0, h0, n0;
                 tile_origin(pt, w0, h0, n0);
                 const int w_l = row % p.Wb, h_l = (row / p.Wb) % p.Hb, n_l = row / (p.Wb * p.Hb);
@@ -542,8 +557,9 @@ tc_igemm3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (lane == 0 && !kInt32) {
             int it = 0;
             for (int item = first_item; item < total_items; item += num_pairs_launched, ++it) {
-                const int ct = item % p.col_tiles;
-                const int pt = (item / p.col_tiles) * 2 + (int)rank;
+                int ct, pair;
+                item_coords(item, ct, pair);
+                const int pt = pair * 2 + (int)rank;
                 const int buf = it % kBufsDiv;
                 if (!mbar_wait(bfull_bar(buf), (uint32_t)(it / kBufsDiv) & 1u, abort_flag, p.status, 8, 0)) break;
                 uint8_t* out_buf = smem_out + buf * Cfg::kTileOut;
