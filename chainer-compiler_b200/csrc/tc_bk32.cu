@@ -4,8 +4,8 @@
 namespace chxq {
 namespace tc {
 
-int launch_tc_bk32(int bn, int epi, const CUtensorMap& tmA, const CUtensorMap& tmB, const TcParams& p, int grid, cudaStream_t s) {
-    return launch_bk<32>(bn, epi, tmA, tmB, p, grid, s);
+int launch_tc_bk32(int bn, int epi, int split, const CUtensorMap& tmA, const CUtensorMap& tmB, const TcParams& p, int grid, cudaStream_t s) {
+    return launch_bk<32>(bn, epi, split, tmA, tmB, p, grid, s);
 }
 
 }  // namespace tc

@@ -256,7 +256,14 @@ int launch_tc_igemm(const TcProblem& q, cudaStream_t s) {
     const int64_t pos_tiles = (int64_t)p.tiles_w * p.tiles_h * p.tiles_n;
     if (q.group_cols > 0 && q.group_cols % 64 != 0)
         return set_error(CHXQ_ERR_UNSUPPORTED, "tensor-core kernel: grouped convolution needs a multiple of 64 output channels per group");
-    const int bn = q.group_cols > 0 ? 64 : (epi_kind == tc::kEpiKGeneric ? 128 : (q.bn ? q.bn : pick_bn(q.cols, pos_tiles)));
+    // Few tiles, many K blocks: clusters that share a tile's K blocks (see tc_igemm_kernel).  At least two blocks per CTA, and all clusters
+    // resident at once.  One B200: ResNet-50 batch 1 op by op 453 -> 351 us, the MLP of 64
+    // rows 66 -> 51 us (with programmatic dependent launch of this kernel, same step).
+    const int64_t num_kb = (int64_t)q.KH * q.KW * (q.c_pad / q.bk), tiles64 = pos_tiles * ((q.cols + 63) / 64);
+    int split = 1;
+    if (chxq::g_variant.load(std::memory_order_relaxed) == 0 && epi_kind != tc::kEpiKGeneric && q.bk >= 64 && q.pool_ho == 0)
+        split = tiles64 * 4 <= num_sms() && num_kb >= 8 ? 4 : (tiles64 * 2 <= num_sms() && num_kb >= 4 ? 2 : 1);
+    const int bn = q.group_cols > 0 || split > 1 ? 64 : (epi_kind == tc::kEpiKGeneric ? 128 : (q.bn ? q.bn : pick_bn(q.cols, pos_tiles)));
     p.col_tiles = (q.cols + bn - 1) / bn;
     const int64_t total_tiles = pos_tiles * p.col_tiles;
     if (total_tiles >= (1ll << 31)) return set_error(CHXQ_ERR_UNSUPPORTED, "tensor-core kernel: too many tiles");
@@ -315,7 +322,7 @@ int launch_tc_igemm(const TcProblem& q, cudaStream_t s) {
                             swizzle_for(q.bk), CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r != CUDA_SUCCESS) return set_error(CHXQ_ERR_CUDA, "cuTensorMapEncodeTiled(B) failed with %d", (int)r);
     }
-    int grid = total_tiles < num_sms() ? (int)total_tiles : num_sms();
+    int grid = split > 1 ? (int)total_tiles * split : (total_tiles < num_sms() ? (int)total_tiles : num_sms());
 
     // Grouped-tile kernel (tc_kernel2.cuh): uint8 epilogues whose outputs (and residual) can move through TMA.
     bool grouped = false, halo = false;
@@ -480,9 +487,9 @@ int launch_tc_igemm(const TcProblem& q, cudaStream_t s) {
                          : tc::launch_tc2_bk64(bn2, epi_kind, q.epi.residual != nullptr, halo, tmA, tmB, tmY, tmR, p, grid, s);
     } else
     switch (q.bk) {
-        case 128: rc = tc::launch_tc_bk128(bn, epi_kind, tmA, tmB, p, grid, s); break;
-        case 64: rc = tc::launch_tc_bk64(bn, epi_kind, tmA, tmB, p, grid, s); break;
-        default: rc = tc::launch_tc_bk32(bn, epi_kind, tmA, tmB, p, grid, s); break;
+        case 128: rc = tc::launch_tc_bk128(bn, epi_kind, split, tmA, tmB, p, grid, s); break;
+        case 64: rc = tc::launch_tc_bk64(bn, epi_kind, split, tmA, tmB, p, grid, s); break;
+        default: rc = tc::launch_tc_bk32(bn, epi_kind, split, tmA, tmB, p, grid, s); break;
     }
     if (g_prof_on) {
         CHXQ_CUDA(cudaEventRecord(rec.e1, s));

@@ -79,6 +79,24 @@ __device__ __forceinline__ void pdl_dependency_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+__device__ __forceinline__ uint32_t cluster_ctarank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+
+// Address of the same shared-memory offset in CTA `rank` of the cluster (a shared::cluster address).
+__device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
+    return r;
+}
+
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 constexpr uint64_t kWaitLimitNs = 2000000000ull;  // 2 s
 
 // Bounded wait.  Returns false when the CTA is aborting (either this wait expired or another did).
@@ -287,7 +305,11 @@ struct TcConfig {
     static constexpr int kSmemBytes = 1024 /*alignment slack*/ + kParamOffset + kParamBytes;
 };
 
-template <int BN, int BK, int EPI>
+// SPLIT > 1: a cluster of SPLIT CTAs works on one tile, each on its share of the K blocks.  The partial accumulators meet in shared memory: CTA
+// r adds up the 16-column chunks c with c % SPLIT == r and runs their epilogue.  Integer sums: the same result whatever the split.
+// Why: a problem with fewer tiles than half the SMs is bound by one CTA's chain of K blocks, 600 to 800 cycles each for one thread that issues
+// the copies (36 blocks of a 3 x 3 layer over 512 channels: 13 us), while most SMs idle.
+template <int BN, int BK, int EPI, int SPLIT = 1>
 __global__ void __launch_bounds__(576, 1)
 tc_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const TcParams p) {
     using Cfg = TcConfig<BN, BK>;
@@ -331,11 +353,24 @@ tc_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_ptr_smem;
+    pdl_launch_dependents();
+    pdl_dependency_wait();  // from here on the previous kernel's output (this kernel's input) is complete and visible
 
     const int pos_tiles = p.tiles_w * p.tiles_h * p.tiles_n;
     const int total_tiles = pos_tiles * p.col_tiles;
     const int taps = p.KH * p.KW;
     const int num_kb = taps * p.c_chunks;
+    static_assert(SPLIT == 1 || (BN == 64 && EPI != kEpiKGeneric), "split K: 64-column tiles");
+    const int split_rank = SPLIT > 1 ? (int)cluster_ctarank() : 0;
+    const int kb_begin = SPLIT > 1 ? split_rank * num_kb / SPLIT : 0, kb_end = SPLIT > 1 ? (split_rank + 1) * num_kb / SPLIT : num_kb;
+    const int first_tile = (int)blockIdx.x / SPLIT, tile_step = (int)gridDim.x / SPLIT;  // split: exactly one tile per cluster
+    // Every thread of the cluster comes by twice, whatever became of its role: before and after the partial sums are read.
+    auto split_sync = [&]() {
+        if constexpr (SPLIT > 1) {
+            __syncwarp();
+            cluster_sync_all();
+        }
+    };
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------
@@ -343,7 +378,7 @@ tc_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
-            for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
+            for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step) {
                 const int ct = tile % p.col_tiles;
                 int pt = tile / p.col_tiles;
                 const int tw = pt % p.tiles_w;
@@ -352,7 +387,7 @@ tc_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 const int tn = pt / p.tiles_h;
                 const int w0 = tw * p.Wb * p.sw - p.pad_left, h0 = th * p.Hb * p.sh - p.pad_top, n0 = tn * p.Nb;
                 const int gbase = p.group_cols > 0 ? (ct * BN / p.group_cols) * p.group_cin : 0;
-                for (int kb = 0; kb < num_kb; ++kb) {
+                for (int kb = kb_begin; kb < kb_end; ++kb) {
                     const int tap = kb / p.c_chunks, cc = kb - tap * p.c_chunks;
                     const int kh = tap / p.KW, kw = tap - kh * p.KW;
                     if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, p.status, 1, 0, p.wait_limit_ns)) {
@@ -371,6 +406,8 @@ tc_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 }
             }
         }
+        split_sync();
+        split_sync();
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
         if (lane == 0) {
@@ -380,13 +417,13 @@ tc_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             bool ok = true;
             const uint32_t desc_hi = kmajor_desc_hi<BK>();
             const uint32_t a_lo0 = kmajor_desc_lo(smem_u32(smem_a)), b_lo0 = kmajor_desc_lo(smem_u32(smem_b));
-            for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++it) {
+            for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step, ++it) {
                 const int acc = it & 1;
                 const uint32_t acc_phase = (uint32_t)(it >> 1) & 1u;
                 if (!mbar_wait(tempty_bar(acc), acc_phase ^ 1u, abort_flag, p.status, 2, 0, p.wait_limit_ns)) break;
                 tc_fence_after();
                 const uint32_t tmem_d = tmem_base + (uint32_t)(acc * BN);
-                for (int kb = 0; kb < num_kb; ++kb) {
+                for (int kb = kb_begin; kb < kb_end; ++kb) {
                     if (!mbar_wait(full_bar(stage), phase, abort_flag, p.status, 3, 0, p.wait_limit_ns)) {
                         ok = false;
                         break;
@@ -396,7 +433,7 @@ tc_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                     const uint32_t b_lo = b_lo0 + (uint32_t)(stage * (Cfg::kStageB >> 4));
 #pragma unroll
                     for (int k = 0; k < BK / 32; ++k)
-                        umma_i8_lohi(tmem_d, a_lo + k * 2, desc_hi, b_lo + k * 2, desc_hi, p.idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                        umma_i8_lohi(tmem_d, a_lo + k * 2, desc_hi, b_lo + k * 2, desc_hi, p.idesc, (kb > kb_begin || k > 0) ? 1u : 0u);
                     umma_commit(empty_bar(stage));  // frees the stage once these MMAs have read it
                     if (++stage == kStages) {
                         stage = 0;
@@ -406,6 +443,8 @@ tc_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 if (ok) umma_commit(tfull_bar(acc));  // accumulator complete
             }
         }
+        split_sync();
+        split_sync();
     } else {
         // ---------------- epilogue warps ----------------
         // Sixteen warps: warp w may touch TMEM lanes 32*(w % 4) .. +31 only, so four warps share each lane quarter and
@@ -425,7 +464,7 @@ tc_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         const RequantParams rq = p.epi.rq;
         const int hi_q = rq.clamp_hi_q >= 0 ? rq.clamp_hi_q : 255;
         int it = 0;
-        for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++it) {
+        for (int tile = first_tile; tile < total_tiles; tile += tile_step, ++it) {
             const int acc = it & 1;
             const uint32_t acc_phase = (uint32_t)(it >> 1) & 1u;
             const int ct = tile % p.col_tiles;
@@ -482,8 +521,8 @@ tc_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 
             uint32_t rowc = 0u;
             if ((EPI == kEpiKInt32 || EPI == kEpiKGeneric) && p.col_mul && row_ok) rowc = row_term(p, no, ho, wo, pos);
-            const bool got = mbar_wait(tfull_bar(acc), acc_phase, abort_flag, p.status, 4, 32, p.wait_limit_ns);
-            if (!__all_sync(0xffffffffu, got)) break;
+            const bool got = __all_sync(0xffffffffu, mbar_wait(tfull_bar(acc), acc_phase, abort_flag, p.status, 4, 32, p.wait_limit_ns));
+            if (SPLIT == 1 && !got) break;
             tc_fence_after();
             const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * BN);
             // One 16-column chunk: registers of TMEM data in, 16 bytes (or 16 int32) out.
@@ -633,6 +672,42 @@ tc_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             // Chunks are processed one after the other, fully unrolled (at most four per warp); the other warps of the
             // scheduler cover the TMEM read latency.
             uint4 resv[4] = {res0, res1, res_load(2), res_load(3)};
+            if constexpr (SPLIT > 1) {
+                // [chunk][4][128 rows] of sixteen bytes over the operand ring, which the finished MMAs have read: conflict-free both ways
+                const uint32_t part = smem_u32(smem_a) + (uint32_t)((sub * 4 * 128 + row) * 16);
+                uint32_t ra[16] = {};
+                if (got) {
+                    tmem_ld_32x32b_x16(taddr + (uint32_t)(sub * 16), ra);
+                    tmem_ld_wait16(ra);
+                    if (sub % SPLIT != split_rank) {
+#pragma unroll
+                        for (int j = 0; j < 4; ++j)
+                            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(part + j * 2048), "r"(ra[4 * j]), "r"(ra[4 * j + 1]),
+                                         "r"(ra[4 * j + 2]), "r"(ra[4 * j + 3])
+                                         : "memory");
+                    }
+                }
+                tc_fence_before();
+                split_sync();
+                if (got && sub % SPLIT == split_rank) {
+#pragma unroll
+                    for (int o = 1; o < SPLIT; ++o) {
+                        const uint32_t peer = map_to_cta(part, (uint32_t)((split_rank + o) % SPLIT));
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            uint4 v;
+                            asm volatile("ld.shared::cluster.v4.b32 {%0, %1, %2, %3}, [%4];"
+                                         : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                                         : "r"(peer + j * 2048)
+                                         : "memory");
+                            ra[4 * j] += v.x; ra[4 * j + 1] += v.y; ra[4 * j + 2] += v.z; ra[4 * j + 3] += v.w;
+                        }
+                    }
+                    process(ra, 0, resv[0]);
+                }
+                split_sync();
+                break;  // one tile per cluster
+            }
 #pragma unroll
             for (int i = 0; i < kMine; ++i) {
                 uint32_t ra[16];
@@ -663,24 +738,58 @@ tc_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     }
 }
 
+// Launch with the programmatic-serialization attribute: the kernel may begin (up to its dependency wait) while the previous
+// kernel in the stream drains.
+template <typename... KArgs, typename... Args>
+cudaError_t launch_pdl_cluster(int cluster, void (*kernel)(KArgs...), int grid, int block, size_t smem, cudaStream_t s, Args&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid, 1, 1);
+    cfg.blockDim = dim3((unsigned)block, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = (unsigned)cluster; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
+template <typename... KArgs, typename... Args>
+cudaError_t launch_pdl(void (*kernel)(KArgs...), int grid, int block, size_t smem, cudaStream_t s, Args&&... args) {
+    return launch_pdl_cluster(1, kernel, grid, block, smem, s, std::forward<Args>(args)...);
+}
+
 // Launches the instantiation for (bn, BK, epi).  Called from the per-BK translation units.
-template <int BN, int BK, int EPI>
+template <int BN, int BK, int EPI, int SPLIT = 1>
 int launch_one(const CUtensorMap& tmA, const CUtensorMap& tmB, const TcParams& p, int grid, cudaStream_t s) {
     using Cfg = TcConfig<BN, BK>;
     static std::atomic<bool> attr_set[64] = {};  // per device; host threads may race here, every writer stores true
     int dev = 0;
     CHXQ_CUDA(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64 || !attr_set[dev].load(std::memory_order_acquire)) {
-        CHXQ_CUDA(cudaFuncSetAttribute(tc_igemm_kernel<BN, BK, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
+        CHXQ_CUDA(cudaFuncSetAttribute(tc_igemm_kernel<BN, BK, EPI, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
         if (dev >= 0 && dev < 64) attr_set[dev].store(true, std::memory_order_release);
     }
-    tc_igemm_kernel<BN, BK, EPI><<<grid, 576, Cfg::kSmemBytes, s>>>(tmA, tmB, p);
-    CHXQ_LAUNCH_CHECK();
+    CHXQ_CUDA(launch_pdl_cluster(SPLIT, tc_igemm_kernel<BN, BK, EPI, SPLIT>, grid, 576, Cfg::kSmemBytes, s, tmA, tmB, p));
+    count_launch(1);
     return CHXQ_OK;
 }
 
 template <int BK>
-int launch_bk(int bn, int epi, const CUtensorMap& tmA, const CUtensorMap& tmB, const TcParams& p, int grid, cudaStream_t s) {
+int launch_bk(int bn, int epi, int split, const CUtensorMap& tmA, const CUtensorMap& tmB, const TcParams& p, int grid, cudaStream_t s) {
+    if constexpr (BK >= 64) {
+        switch (split * 4 + epi) {
+            case 2 * 4 + kEpiKInt32: return launch_one<64, BK, kEpiKInt32, 2>(tmA, tmB, p, grid, s);
+            case 2 * 4 + kEpiKU8: return launch_one<64, BK, kEpiKU8, 2>(tmA, tmB, p, grid, s);
+            case 2 * 4 + kEpiKU8Fold: return launch_one<64, BK, kEpiKU8Fold, 2>(tmA, tmB, p, grid, s);
+            case 4 * 4 + kEpiKInt32: return launch_one<64, BK, kEpiKInt32, 4>(tmA, tmB, p, grid, s);
+            case 4 * 4 + kEpiKU8: return launch_one<64, BK, kEpiKU8, 4>(tmA, tmB, p, grid, s);
+            case 4 * 4 + kEpiKU8Fold: return launch_one<64, BK, kEpiKU8Fold, 4>(tmA, tmB, p, grid, s);
+        }
+    }
     if (epi == kEpiKGeneric) return launch_one<128, BK, kEpiKGeneric>(tmA, tmB, p, grid, s);  // rare path: one tile shape
     switch (bn * 4 + epi) {
         case 64 * 4 + kEpiKInt32: return launch_one<64, BK, kEpiKInt32>(tmA, tmB, p, grid, s);

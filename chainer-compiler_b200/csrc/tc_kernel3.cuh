@@ -23,24 +23,6 @@
 namespace chxq {
 namespace tc {
 
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-
-// Address of the same shared-memory offset in CTA `rank` of the cluster (a shared::cluster address).
-__device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
-    return r;
-}
-
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
 // Arrival on a barrier that may live in the partner CTA.  Default semantics (release at CTA scope): what the arrival orders here
 // are tensor-memory reads, which tcgen05.fence::before_thread_sync covers; a cluster-scope release would cost a memory barrier
 // per warp and item.

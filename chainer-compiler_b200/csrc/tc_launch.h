@@ -79,9 +79,10 @@ constexpr int kEpiKU8 = 1;       // requantize to uint8, optional residual tail
 constexpr int kEpiKGeneric = 2;  // int8 output and/or a weight zero-point term: general requantization
 constexpr int kEpiKU8Fold = 3;   // uint8 with one folded multiplier per channel (RequantParams::fold)
 
-int launch_tc_bk32(int bn, int epi, const CUtensorMap& tmA, const CUtensorMap& tmB, const TcParams& p, int grid, cudaStream_t s);
-int launch_tc_bk64(int bn, int epi, const CUtensorMap& tmA, const CUtensorMap& tmB, const TcParams& p, int grid, cudaStream_t s);
-int launch_tc_bk128(int bn, int epi, const CUtensorMap& tmA, const CUtensorMap& tmB, const TcParams& p, int grid, cudaStream_t s);
+// split: CTAs that share one tile's K blocks (1, 2 or 4; above 1: 64-column tiles, grid = tiles x split).
+int launch_tc_bk32(int bn, int epi, int split, const CUtensorMap& tmA, const CUtensorMap& tmB, const TcParams& p, int grid, cudaStream_t s);
+int launch_tc_bk64(int bn, int epi, int split, const CUtensorMap& tmA, const CUtensorMap& tmB, const TcParams& p, int grid, cudaStream_t s);
+int launch_tc_bk128(int bn, int epi, int split, const CUtensorMap& tmA, const CUtensorMap& tmB, const TcParams& p, int grid, cudaStream_t s);
 // Grouped-tile kernel (tc_kernel2.cuh); bn is 64 or 128, epi is kEpiKU8 or kEpiKU8Fold.
 // pool: the fused max-pooling form (bn 64, no residual; 64-byte K tiles only), with or without halo tiles.
 int launch_tc2_bk64_pool(int epi, bool halo, const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmY, const CUtensorMap& tmR, const TcParams& p,
