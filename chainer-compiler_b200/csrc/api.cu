@@ -8,6 +8,7 @@
 
 #include "common.h"
 #include "kernels.h"
+#include "pdl.cuh"
 
 namespace chxq {
 namespace {
@@ -57,13 +58,13 @@ __device__ __forceinline__ uint32_t load4_unaligned(const uint8_t* p, int64_t n)
 // launch in front and global atomics.  A tile: 32-bit loads along N at any alignment of the rows, a 4 x 4 byte transpose in registers, the
 // tile through shared memory as words with a pitch of 17 (conflict-free), 128-bit stores along K.
 constexpr int kTrSplit = 8;
-__global__ void __cluster_dims__(1, kTrSplit, 1) __launch_bounds__(256) transpose_b_terms_kernel(
-        const uint8_t* __restrict__ b, int64_t K, int64_t N, int64_t k_pad, uint8_t* __restrict__ bt, ZpSpec za, int a_signed, int b_signed,
-        int32_t* __restrict__ T, ZpSpec zb, int32_t* __restrict__ zbn) {
+__device__ __forceinline__ void transpose_b_terms(
+        int64_t col_block, int split, const uint8_t* __restrict__ b, int64_t K, int64_t N, int64_t k_pad, uint8_t* __restrict__ bt, const ZpSpec& za,
+        int a_signed, int b_signed, int32_t* __restrict__ T, const ZpSpec& zb, int32_t* __restrict__ zbn) {
     __shared__ uint32_t tw[2][64][17];
     __shared__ int colsum[64];
     const int tid = threadIdx.x;
-    const int64_t n0 = (int64_t)blockIdx.x * 64;
+    const int64_t n0 = col_block * 64;
     const int a = tid / 16, bq = tid % 16;   // load side: rows k0 + 4a .. +3, columns n0 + 4bq .. +3
     const int col = tid / 4, q = tid % 4;    // store side: column n0 + col, rows k0 + 16q .. +15
     const bool words_ok = (N % 4 == 0) && ((reinterpret_cast<uintptr_t>(b) & 3u) == 0);
@@ -71,29 +72,43 @@ __global__ void __cluster_dims__(1, kTrSplit, 1) __launch_bounds__(256) transpos
     const int64_t k_tiles = (k_pad + 63) / 64;
     const int64_t n = n0 + 4 * bq;
     int part[4] = {0, 0, 0, 0};
+    // (a row's bytes are aligned words shifted together; loads are predicated, not branched around, so that all of a tile's are in flight)
     auto load = [&](int64_t kt, uint32_t (&r)[4]) {
+        const int64_t k0 = kt * 64 + 4 * a;
+        const int rows = kt < k_tiles && n < N && k0 < K ? (int)min((int64_t)4, K - k0) : 0;
+        if (words_ok) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) r[i] = i < rows ? __ldg(reinterpret_cast<const uint32_t*>(b + (k0 + i) * N + n)) : 0u;
+            return;
+        }
+        const int left = (int)min((int64_t)4, N - n);
+        uint32_t lo[4], hi[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const int64_t k = kt * 64 + 4 * a + i;
-            uint32_t v = 0u;
-            if (kt < k_tiles && k < K && n < N) {
-                const uint8_t* src = b + k * N + n;
-                v = words_ok ? __ldg(reinterpret_cast<const uint32_t*>(src)) : load4_unaligned(src, N - n);
-            }
-            r[i] = v;
+            const uintptr_t addr = reinterpret_cast<uintptr_t>(b) + (uintptr_t)((k0 + i) * N + n);
+            const uint32_t* w = reinterpret_cast<const uint32_t*>(addr & ~(uintptr_t)3u);
+            lo[i] = i < rows ? __ldg(w) : 0u;
+            hi[i] = i < rows && left > 4 - (int)(addr & 3u) ? __ldg(w + 1) : 0u;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uintptr_t addr = reinterpret_cast<uintptr_t>(b) + (uintptr_t)((k0 + i) * N + n);
+            const uint32_t v = __funnelshift_r(lo[i], hi[i], 8 * (int)(addr & 3u));
+            r[i] = left >= 4 ? v : v & ((1u << (8 * left)) - 1u);
         }
     };
+    const int z_all = T != nullptr && za.len == 1 ? zp_at(za, 0, a_signed) : 0;
     uint32_t r[4];
-    load(blockIdx.y, r);
+    load(split, r);
     int buf = 0;
-    for (int64_t kt = blockIdx.y; kt < k_tiles; kt += kTrSplit, buf ^= 1) {
+    for (int64_t kt = split; kt < k_tiles; kt += kTrSplit, buf ^= 1) {
         uint32_t next[4];
         load(kt + kTrSplit, next);
         if (T != nullptr) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const int64_t k = kt * 64 + 4 * a + i;
-                const int z = k < K ? zp_at(za, k, a_signed) : 0;
+                const int z = za.len == 1 ? z_all : (k < K ? zp_at(za, k, a_signed) : 0);
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const uint32_t byte = (r[i] >> (8 * j)) & 0xffu;
@@ -129,14 +144,15 @@ __global__ void __cluster_dims__(1, kTrSplit, 1) __launch_bounds__(256) transpos
         }
         cluster.sync();  // a block's shared memory stays until it has been read
     }
-    if (zbn != nullptr && blockIdx.y == 0 && tid < 64 && n0 + tid < N) zbn[n0 + tid] = zp_at(zb, n0 + tid, b_signed);
+    if (zbn != nullptr && split == 0 && tid < 64 && n0 + tid < N) zbn[n0 + tid] = zp_at(zb, n0 + tid, b_signed);
 }
 
 // One warp per row of A: R[m] = sum_k (a[m, k] - za[k]) (absent: null), and the row at a pitch TMA can describe (K rounded up to sixteen
 // bytes, zero padded; absent: null).  Sixteen bytes per lane, read as aligned words at whatever address the row starts.
-__global__ void __launch_bounds__(256) gemm_a_rows_kernel(
-        const uint8_t* __restrict__ a, int a_signed, int64_t M, int64_t K, ZpSpec za, int64_t pitch, uint8_t* __restrict__ out, int32_t* __restrict__ R) {
-    const int64_t m = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+__device__ __forceinline__ void gemm_a_rows(
+        int64_t block, const uint8_t* __restrict__ a, int a_signed, int64_t M, int64_t K, const ZpSpec& za, int64_t pitch, uint8_t* __restrict__ out,
+        int32_t* __restrict__ R) {
+    const int64_t m = (block * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (m >= M) return;
     const uint8_t* row = a + m * K;
@@ -163,6 +179,31 @@ __global__ void __launch_bounds__(256) gemm_a_rows_kernel(
     if (lane == 0) R[m] = za.len == 1 ? s - (int)K * zp_at(za, 0, a_signed) : s;
 }
 
+// Both, as one launch: clusters [0, col_blocks) take the columns of B, the blocks after them the rows of A where those need a pass.
+struct GemmPrep {
+    const uint8_t* a;
+    const uint8_t* b;
+    int64_t M, N, K, k_pad, a_pitch;
+    int a_signed, b_signed;
+    ZpSpec za, zb;
+    uint8_t* bt;
+    int32_t* T;
+    int32_t* zbn;
+    uint8_t* a_copy;
+    int32_t* R;
+    int64_t col_blocks;
+};
+
+__global__ void __cluster_dims__(kTrSplit, 1, 1) __launch_bounds__(256) gemm_prep_kernel(const GemmPrep g) {
+    pdl_launch_dependents();
+    pdl_dependency_wait();
+    const int64_t cluster = blockIdx.x / kTrSplit;
+    if (cluster < g.col_blocks)
+        transpose_b_terms(cluster, (int)(blockIdx.x % kTrSplit), g.b, g.K, g.N, g.k_pad, g.bt, g.za, g.a_signed, g.b_signed, g.T, g.zb, g.zbn);
+    else
+        gemm_a_rows((int64_t)blockIdx.x - g.col_blocks * kTrSplit, g.a, g.a_signed, g.M, g.K, g.za, g.a_pitch, g.a_copy, g.R);
+}
+
 // Everything a convolution over NCHW maps (or with a device-resident zero point) needs in front of the tensor-core kernel, as one launch.
 // Blocks [0, M): one output channel each -- its weights from OIHW to the K-major row [tap * c_pitch + c] (zero padded), their sum times the
 // activation zero point, and its own zero point widened.  The other blocks: 128 positions of the input map each, transposed to NHWC rows of
@@ -172,7 +213,7 @@ __global__ void __launch_bounds__(256) gemm_a_rows_kernel(
 // Bound: one read and one write of the map.  Transpose and packing were four launches with a byte-wise path for maps whose extent is no
 // multiple of four; a padded map with a zero point went through an im2col matrix, KH * KW times the bytes, and a map with a device zero
 // point through the one-thread-per-output CUDA-core kernel.  One B200: the dynamically quantized
-// 3 x 3 convolution of [8, 64, 56, 56], four operators, 1186 -> 45 us; the pass itself 13.6 us for 25.7 MB in and out.
+// 3 x 3 convolution of [8, 64, 56, 56], four operators, 1186 -> 28 us; the pass itself 13.5 us for 25.7 MB in and out.
 struct ConvPrep {
     const uint8_t* x;
     const uint8_t* w;
@@ -200,6 +241,8 @@ __global__ void __launch_bounds__(256) conv_prep_kernel(const ConvPrep a) {
     __shared__ __align__(16) uint32_t tw[16 * kPrepPitch];  // [channel quad][position]: four channels of a position per word
     __shared__ int warp_sum[8];
     const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+    pdl_launch_dependents();
+    pdl_dependency_wait();
     const int zx = a.x_zp_dev ? ldq_rt(a.x_zp_dev, 0, a.x_signed) : a.x_zp;
     if ((int)blockIdx.x < a.M) {
         const int m = blockIdx.x;
@@ -250,34 +293,65 @@ __global__ void __launch_bounds__(256) conv_prep_kernel(const ConvPrep a) {
     const int c_first = part * a.tiles_per_part * 64, c_end = min(a.cs, c_first + a.tiles_per_part * 64);
     for (int c0 = c_first; c0 < c_end; c0 += 64) {
         if (!kNhwc) {
+            // predicated loads, not branched around: all of a thread's are in flight together
             uint32_t r[2][4];
+            const uint8_t* base = a.x + (int64_t)n * a.C * HW;
+            const int ch0 = c0 + 4 * warp;
+            if (words) {
 #pragma unroll
-            for (int h = 0; h < 2; ++h)
+                for (int h = 0; h < 2; ++h)
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int ch = c0 + 4 * (warp + 8 * h) + i;
-                    uint32_t v = 0u;
-                    if (ch < a.C && lp < plane) {
-                        const uint8_t* src = a.x + ((int64_t)n * a.C + ch) * HW;
-                        if (words) {
-                            v = __ldg(reinterpret_cast<const uint32_t*>(src + lp));
-                        } else if (run) {
-                            v = load4_unaligned(src + run_off, kBorder ? 4 : HW - lp);
-                        } else {
-                            int y = lh, x = lw;
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) {
-                                const bool in = y >= 0 && y < a.H && x >= 0 && x < a.W;
-                                if (lp + j < plane) v |= (in ? (uint32_t)src[(int64_t)y * a.W + x] : (uint32_t)zx & 0xffu) << (8 * j);
-                                if (++x + a.pl == a.Wp) {
-                                    x = -a.pl;
-                                    ++y;
-                                }
-                            }
-                        }
+                    for (int i = 0; i < 4; ++i) {
+                        const int ch = ch0 + 32 * h + i;
+                        r[h][i] = ch < a.C && run ? __ldg(reinterpret_cast<const uint32_t*>(base + (int64_t)ch * HW + lp)) : 0u;
                     }
-                    r[h][i] = v;
+            } else if (run) {
+                const int left = kBorder ? 4 : min(4, HW - lp);
+                uint32_t hi[2][4];
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const int ch = ch0 + 32 * h + i;
+                        const uintptr_t addr = reinterpret_cast<uintptr_t>(base) + (uintptr_t)((int64_t)ch * HW + run_off);
+                        const uint32_t* w = reinterpret_cast<const uint32_t*>(addr & ~(uintptr_t)3u);
+                        r[h][i] = ch < a.C ? __ldg(w) : 0u;
+                        hi[h][i] = ch < a.C && left > 4 - (int)(addr & 3u) ? __ldg(w + 1) : 0u;
+                    }
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const uintptr_t addr = reinterpret_cast<uintptr_t>(base) + (uintptr_t)((int64_t)(ch0 + 32 * h + i) * HW + run_off);
+                        const uint32_t v = __funnelshift_r(r[h][i], hi[h][i], 8 * (int)(addr & 3u));
+                        r[h][i] = left >= 4 ? v : v & ((1u << (8 * left)) - 1u);
+                    }
+            } else {
+                int off[4];  // of the four positions; -1: border, -2: past the map
+                int y = lh, x = lw;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    off[j] = lp + j >= plane ? -2 : (y >= 0 && y < a.H && x >= 0 && x < a.W ? y * a.W + x : -1);
+                    if (++x + a.pl == a.Wp) {
+                        x = -a.pl;
+                        ++y;
+                    }
                 }
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const int ch = ch0 + 32 * h + i;
+                        uint32_t v = 0u;
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            uint32_t byte = off[j] == -1 && ch < a.C ? (uint32_t)zx & 0xffu : 0u;
+                            if (off[j] >= 0 && ch < a.C) byte = __ldg(base + (int64_t)ch * HW + off[j]);
+                            v |= byte << (8 * j);
+                        }
+                        r[h][i] = v;
+                    }
+            }
             if (c0 != c_first) __syncthreads();  // the previous channel tile has been read
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
@@ -331,17 +405,19 @@ __global__ void __launch_bounds__(256) conv_prep_kernel(const ConvPrep a) {
 
 int launch_conv_prep(const ConvPrep& a, cudaStream_t s) {
     const unsigned grid = (unsigned)((int64_t)a.pos_tiles * a.N * a.parts + a.M);
+    cudaError_t e;
     switch ((a.x_nhwc ? 4 : 0) + (a.border ? 2 : 0) + (a.pix ? 1 : 0)) {
-        case 0: conv_prep_kernel<false, false, false><<<grid, 256, 0, s>>>(a); break;
-        case 1: conv_prep_kernel<false, false, true><<<grid, 256, 0, s>>>(a); break;
-        case 2: conv_prep_kernel<false, true, false><<<grid, 256, 0, s>>>(a); break;
-        case 3: conv_prep_kernel<false, true, true><<<grid, 256, 0, s>>>(a); break;
-        case 4: conv_prep_kernel<true, false, false><<<grid, 256, 0, s>>>(a); break;
-        case 5: conv_prep_kernel<true, false, true><<<grid, 256, 0, s>>>(a); break;
-        case 6: conv_prep_kernel<true, true, false><<<grid, 256, 0, s>>>(a); break;
-        default: conv_prep_kernel<true, true, true><<<grid, 256, 0, s>>>(a); break;
+        case 0: e = launch_pdl(conv_prep_kernel<false, false, false>, (int)grid, 256, 0, s, a); break;
+        case 1: e = launch_pdl(conv_prep_kernel<false, false, true>, (int)grid, 256, 0, s, a); break;
+        case 2: e = launch_pdl(conv_prep_kernel<false, true, false>, (int)grid, 256, 0, s, a); break;
+        case 3: e = launch_pdl(conv_prep_kernel<false, true, true>, (int)grid, 256, 0, s, a); break;
+        case 4: e = launch_pdl(conv_prep_kernel<true, false, false>, (int)grid, 256, 0, s, a); break;
+        case 5: e = launch_pdl(conv_prep_kernel<true, false, true>, (int)grid, 256, 0, s, a); break;
+        case 6: e = launch_pdl(conv_prep_kernel<true, true, false>, (int)grid, 256, 0, s, a); break;
+        default: e = launch_pdl(conv_prep_kernel<true, true, true>, (int)grid, 256, 0, s, a); break;
     }
-    CHXQ_LAUNCH_CHECK();
+    CHXQ_CUDA(e);
+    count_launch(1);
     return CHXQ_OK;
 }
 
@@ -624,7 +700,9 @@ struct GemmWs {
 
 GemmWs gemm_ws_layout(int64_t M, int64_t N, int64_t K) {
     GemmWs w;
-    w.bk = choose_bk((int)(K > (1 << 20) ? 128 : K));
+    // Ragged K: 128-byte K tiles from 513 on even where 64 would pad less (at most an eighth of the weights) -- half the copies and barrier
+    // round trips per byte, and the CTA-pair kernel.
+    w.bk = K % 16 != 0 && K > 512 ? 128 : choose_bk((int)(K > (1 << 20) ? 128 : K));
     w.k_pad = (K + w.bk - 1) / w.bk * w.bk;
     size_t off = 0;
     w.bt_off = off; off += align_up((size_t)N * (size_t)w.k_pad, 256);
@@ -645,7 +723,7 @@ bool gemm_tc_eligible(const void* a, int64_t M, int64_t N, int64_t K) {
 
 // Rows of A that do not start on sixteen-byte boundaries (K % 16 != 0) reach the tensor cores through a copy at a wider pitch.  The copy
 // is one pass over A; the CUDA-core kernel makes one multiply-add per lane and clock.  One B200, whole calls: 509 x 3073 x 1283 with zero
-// points 293 -> 41 us, the 784-1000-1000-10 MLP of 64 rows (two of its three products have K = 1000) 103.5 -> 66 us.
+// points 293 -> 22 us, the 784-1000-1000-10 MLP of 64 rows (two of its three products have K = 1000) 104 -> 39 us.
 bool gemm_tc_via_copy(int64_t M, int64_t N, int64_t K) {
     return K % 16 != 0 && K >= 16 && M >= 1 && N >= 1 && M < (1ll << 31) && N < (1ll << 31) && K < (1ll << 20);
 }
@@ -682,14 +760,13 @@ int gemm_dispatch(
         const uint8_t* ab = static_cast<const uint8_t*>(a) + bi * M * K;
         const uint8_t* bb = static_cast<const uint8_t*>(b) + bi * K * N;
         if ((ws.k_pad + 63) / 64 > 65535) return set_error(CHXQ_ERR_UNSUPPORTED, "%s: K too large for the tensor-core path", op);
-        if (a_copy != nullptr || R != nullptr) {
-            gemm_a_rows_kernel<<<blocks_for(M * 32), 256, 0, s>>>(ab, a_signed ? 1 : 0, M, K, za, ws.a_pitch, a_copy, R);
-            CHXQ_LAUNCH_CHECK();
-        }
-        // one pass over B: the K-major copy, the column terms of a's zero point and b's zero points widened
-        transpose_b_terms_kernel<<<dim3((unsigned)((N + 63) / 64), kTrSplit), 256, 0, s>>>(bb, K, N, ws.k_pad, bt, za, a_signed ? 1 : 0,
-                                                                                           b_signed ? 1 : 0, T, zb, zbn);
-        CHXQ_LAUNCH_CHECK();
+        // one launch: B K-major, the column terms of a's zero point, b's zero points widened, and what A needs
+        GemmPrep g{ab, bb, M, N, K, ws.k_pad, ws.a_pitch, a_signed ? 1 : 0, b_signed ? 1 : 0, za, zb, bt, T, zbn, a_copy, R, (N + 63) / 64};
+        const int64_t row_blocks = a_copy != nullptr || R != nullptr ? ((M + 7) / 8 + kTrSplit - 1) / kTrSplit * kTrSplit : 0;
+        const int64_t blocks = g.col_blocks * kTrSplit + row_blocks;
+        if (blocks >= (1ll << 31)) return set_error(CHXQ_ERR_UNSUPPORTED, "%s: too many blocks in the repacking grid", op);
+        CHXQ_CUDA(launch_pdl(gemm_prep_kernel, (int)blocks, 256, 0, s, g));
+        count_launch(1);
         TcProblem p{};
         p.a = a_copy ? a_copy : ab; p.a_signed = a_signed; p.C = (int)K; p.a_cs = ws.a_pitch; p.W = (int)M; p.H = 1; p.N = 1;
         p.b = bt; p.b_signed = b_signed; p.cols = (int)N; p.c_pad = (int)ws.k_pad; p.bk = ws.bk;

@@ -23,6 +23,7 @@
 
 #include "common.h"
 #include "kernels.h"
+#include "pdl.cuh"
 #include "tc_launch.h"
 
 namespace chxq {
@@ -65,18 +66,6 @@ __device__ __forceinline__ uint64_t global_timer_ns() {
     uint64_t t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
-}
-
-// Programmatic dependent launch: a kernel launched with the programmatic-serialization attribute may start while the kernel
-// before it in the stream is still running.  launch_dependents lets the next kernel's CTAs be scheduled as soon as this
-// kernel's CTAs leave their SMs; dependency_wait blocks until the previous kernel has completed and its writes are visible.
-// Everything a CTA does before dependency_wait (barrier initialisation, tensor-memory allocation) overlaps the previous
-// kernel's tail; nothing before it may touch global memory that the previous kernel writes or reads.
-__device__ __forceinline__ void pdl_launch_dependents() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-__device__ __forceinline__ void pdl_dependency_wait() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
@@ -736,30 +725,6 @@ tc_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         tc_fence_after();
         tmem_dealloc(tmem_base, Cfg::kTmemCols);
     }
-}
-
-// Launch with the programmatic-serialization attribute: the kernel may begin (up to its dependency wait) while the previous
-// kernel in the stream drains.
-template <typename... KArgs, typename... Args>
-cudaError_t launch_pdl_cluster(int cluster, void (*kernel)(KArgs...), int grid, int block, size_t smem, cudaStream_t s, Args&&... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid, 1, 1);
-    cfg.blockDim = dim3((unsigned)block, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    at[1].id = cudaLaunchAttributeClusterDimension;
-    at[1].val.clusterDim.x = (unsigned)cluster; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
-    cfg.numAttrs = cluster > 1 ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
-}
-
-template <typename... KArgs, typename... Args>
-cudaError_t launch_pdl(void (*kernel)(KArgs...), int grid, int block, size_t smem, cudaStream_t s, Args&&... args) {
-    return launch_pdl_cluster(1, kernel, grid, block, smem, s, std::forward<Args>(args)...);
 }
 
 // Launches the instantiation for (bn, BK, epi).  Called from the per-BK translation units.
