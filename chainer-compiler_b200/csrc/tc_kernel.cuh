@@ -2,8 +2,8 @@
 // TMEM (kind::i8), operands staged in shared memory by TMA (no cluster multicast anywhere), zero-point terms,
 // per-channel requantize, bias, ReLU clamp and the residual tail applied in the epilogue straight out of TMEM.
 //
-// One persistent CTA per SM, 576 threads:
-//   warp 0      : TMA producer (one elected lane): A box {bk, Wb, Hb, Nb} of an NHWC map / matrix,
+// One persistent CTA per SM, 608 threads:
+//   warps 0, 18 : TMA producers (one elected lane each): A box {bk, Wb, Hb, Nb} of an NHWC map / matrix,
 //                 B box {bk, BN} of the packed weights, ring of kStages shared-memory stages.
 //   warp 1      : allocates TMEM, issues tcgen05.mma (one elected lane), M = 128, N = BN, K = 32 per
 //                 instruction; accumulators are double-buffered in TMEM (2 x BN columns) so the
@@ -279,6 +279,28 @@ __device__ __forceinline__ void store_nchw16(const TcParams& p, int64_t pos, int
         if (j < n) yo[j * p.y_plane] = (int32_t)r[j];
 }
 
+// Stores sixteen columns of thirty-two consecutive positions (lane l holds position l's) as int32 rows at any alignment: each half of the warp
+// transposes its 16 x 16 block (four butterfly steps), so that a store covers 64 consecutive bytes of two rows instead of four bytes of
+// thirty-two.  first: the position of this half's lane 0; called by the whole warp, positions from p.Wo on are not stored.
+__device__ __forceinline__ void store_rows16(const TcParams& p, int64_t first, int cbase, int lane, uint32_t (&r)[16]) {
+#pragma unroll
+    for (int s = 8; s >= 1; s /= 2) {
+        const bool up = (lane & s) != 0;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            if (j & s) continue;
+            const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? r[j] : r[j + s], s);
+            if (up) r[j] = got;
+            else r[j + s] = got;
+        }
+    }
+    const int c = cbase + (lane & 15);
+    int32_t* yo = static_cast<int32_t*>(p.y) + first * p.ldc + c;
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+        if (c < p.cols && first + j < p.Wo) yo[j * p.ldc] = (int32_t)r[j];
+}
+
 template <int BN, int BK>
 struct TcConfig {
     static constexpr int kStageA = 128 * BK;
@@ -299,7 +321,7 @@ struct TcConfig {
 // Why: a problem with fewer tiles than half the SMs is bound by one CTA's chain of K blocks, 600 to 800 cycles each for one thread that issues
 // the copies (36 blocks of a 3 x 3 layer over 512 channels: 13 us), while most SMs idle.
 template <int BN, int BK, int EPI, int SPLIT = 1>
-__global__ void __launch_bounds__(576, 1)
+__global__ void __launch_bounds__(608, 1)
 tc_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const TcParams p) {
     using Cfg = TcConfig<BN, BK>;
     constexpr int kStages = Cfg::kStages;
@@ -323,7 +345,7 @@ tc_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
-            mbar_init(full_bar(s), 1);
+            mbar_init(full_bar(s), 2);  // one arrival per producer, each announcing its own bytes
             mbar_init(empty_bar(s), 1);
         }
         for (int a = 0; a < 2; ++a) {
@@ -361,8 +383,10 @@ tc_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         }
     };
 
-    if (warp == 0) {
-        // ---------------- TMA producer ----------------
+    if (warp == 0 || warp == 18) {
+        // ---------------- TMA producers: warp 0 the positions, warp 18 the weights (a thread is held 300 to 400 cycles per copy; one
+        // thread for both operands paced the whole main loop) ----------------
+        const bool is_a = warp == 0;
         if (lane == 0) {
             int stage = 0;
             uint32_t phase = 0;
@@ -383,11 +407,15 @@ tc_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                         ok = false;
                         break;
                     }
-                    mbar_expect_tx(full_bar(stage), Cfg::kStageBytes);
-                    tma_load_4d(smem_u32(smem_a + stage * Cfg::kStageA), &tmA, full_bar(stage), gbase + cc * BK, w0 + kw, h0 + kh, n0);
-                    // (test of the bounded waits only: one weight load left out, so that this stage never fills)
-                    if (kb != p.test_skip_kb)
-                        tma_load_2d(smem_u32(smem_b + stage * Cfg::kStageB), &tmB, full_bar(stage), tap * p.c_pad + cc * BK, ct * BN);
+                    if (is_a) {
+                        mbar_expect_tx(full_bar(stage), Cfg::kStageA);
+                        tma_load_4d(smem_u32(smem_a + stage * Cfg::kStageA), &tmA, full_bar(stage), gbase + cc * BK, w0 + kw, h0 + kh, n0);
+                    } else {
+                        mbar_expect_tx(full_bar(stage), Cfg::kStageB);
+                        // (test of the bounded waits only: one weight load left out, so that this stage never fills)
+                        if (kb != p.test_skip_kb)
+                            tma_load_2d(smem_u32(smem_b + stage * Cfg::kStageB), &tmB, full_bar(stage), tap * p.c_pad + cc * BK, ct * BN);
+                    }
                     if (++stage == kStages) {
                         stage = 0;
                         phase ^= 1u;
@@ -518,7 +546,10 @@ tc_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             auto process = [&](uint32_t (&r)[16], const int i, const uint4 resv) {
                 const int ch = i * 4 + sub;
                 const int cbase = col0 + ch * 16;
-                if (!(row_ok && cbase < p.cols)) return;
+                if (cbase >= p.cols) return;  // warp-uniform
+                // int32 rows that do not start on sixteen-byte boundaries, positions in flat order: the warp stores together (store_rows16)
+                const bool rows16 = EPI == kEpiKInt32 && !p.vec_ok && p.y_plane == 0 && p.Wb == 128;
+                if (!row_ok && !rows16) return;
                 const bool full_chunk = cbase + 16 <= p.cols;
                 const int64_t o = pos * p.ldc + cbase;
                 const float4* pm = reinterpret_cast<const float4*>(s_mult + i * 16);
@@ -548,7 +579,9 @@ tc_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 }
                 if (EPI == kEpiKInt32) {
                     int32_t* yo = static_cast<int32_t*>(p.y) + o;
-                    if (p.y_plane > 0) {
+                    if (rows16) {
+                        store_rows16(p, pos - (lane & 15), cbase, lane, r);
+                    } else if (p.y_plane > 0) {
                         store_nchw16(p, pos, cbase, p.cols - cbase, r);
                     } else if (full_chunk && p.vec_ok) {
 #pragma unroll
@@ -738,7 +771,7 @@ int launch_one(const CUtensorMap& tmA, const CUtensorMap& tmB, const TcParams& p
         CHXQ_CUDA(cudaFuncSetAttribute(tc_igemm_kernel<BN, BK, EPI, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
         if (dev >= 0 && dev < 64) attr_set[dev].store(true, std::memory_order_release);
     }
-    CHXQ_CUDA(launch_pdl_cluster(SPLIT, tc_igemm_kernel<BN, BK, EPI, SPLIT>, grid, 576, Cfg::kSmemBytes, s, tmA, tmB, p));
+    CHXQ_CUDA(launch_pdl_cluster(SPLIT, tc_igemm_kernel<BN, BK, EPI, SPLIT>, grid, 608, Cfg::kSmemBytes, s, tmA, tmB, p));
     count_launch(1);
     return CHXQ_OK;
 }
