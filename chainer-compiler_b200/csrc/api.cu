@@ -1027,10 +1027,12 @@ struct PrepPlan {
     size_t blob_off, x_off, pix_off, y_off, total;
 };
 
-bool prep_plan(const chxq_conv_geom& g, int y_elem, bool border, bool pixel_sums, PrepPlan* out) {
+// border: a border of the zero point is needed where the convolution pads; copy: the map is written anew (false: an NHWC map that the
+// tensor-core kernel reads as it is -- the launch prepares the weights alone).
+bool prep_plan(const chxq_conv_geom& g, int y_elem, bool border, bool pixel_sums, PrepPlan* out, bool copy = true) {
     if (g.group != 1 || g.stride_h > 8 || g.stride_w > 8 || g.pad_top < 0 || g.pad_left < 0 || g.pad_bottom < 0 || g.pad_right < 0) return false;
     const bool padded = g.pad_top || g.pad_left || g.pad_bottom || g.pad_right;
-    border = padded && (border || g.pad_top >= g.KH || g.pad_left >= g.KW);
+    border = copy && padded && (border || g.pad_top >= g.KH || g.pad_left >= g.KW);
     const int64_t Hp = g.H + (border ? g.pad_top + g.pad_bottom : 0), Wp = g.W + (border ? g.pad_left + g.pad_right : 0);
     const int taps = g.KH * g.KW;
     PrepPlan& P = *out;
@@ -1041,7 +1043,7 @@ bool prep_plan(const chxq_conv_geom& g, int y_elem, bool border, bool pixel_sums
     if (border) P.g.pad_top = P.g.pad_left = P.g.pad_bottom = P.g.pad_right = 0;
     ConvPrep& a = P.prep;
     a.cs = (g.C + 15) / 16 * 16;
-    P.g.x_cstride = a.cs;
+    if (copy) P.g.x_cstride = a.cs;
     const bool y_nchw = g.y_layout == CHXQ_NCHW;
     if (y_nchw) {
         P.g.y_layout = CHXQ_NHWC;
@@ -1057,7 +1059,7 @@ bool prep_plan(const chxq_conv_geom& g, int y_elem, bool border, bool pixel_sums
     a.border = border; a.pt = border ? g.pad_top : 0; a.pl = border ? g.pad_left : 0;
     a.Hp = (int)Hp; a.Wp = (int)Wp;
     a.c_pitch = P.pl.c_pitch; a.k_total = P.pl.k_total;
-    a.pos_tiles = (int)((Hp * Wp + kPrepPos - 1) / kPrepPos);
+    a.pos_tiles = copy ? (int)((Hp * Wp + kPrepPos - 1) / kPrepPos) : 0;
     // Channel tiles side by side where nothing is summed over them; with pixel sums a block keeps its channels, in up to four shares
     // (each is another load per tap in the epilogue) where the positions alone leave SMs idle.
     const int c_tiles = (a.cs + 63) / 64;
@@ -1075,7 +1077,8 @@ bool prep_plan(const chxq_conv_geom& g, int y_elem, bool border, bool pixel_sums
     size_t off = 0;
     P.blob_off = off; off += L.pack_total;
     off = align_up(off, 1024);
-    P.x_off = off; off += align_up((size_t)g.N * (size_t)(Hp * Wp) * a.cs, 1024);
+    P.x_off = off;
+    if (copy) off += align_up((size_t)g.N * (size_t)(Hp * Wp) * a.cs, 1024);
     P.pix_off = off;
     if (pixel_sums) off += align_up((size_t)a.parts * g.N * (size_t)(Hp * Wp) * 4, 1024);
     P.y_off = off;
@@ -1105,7 +1108,11 @@ int conv_prep_run(const void* x, const void* w, const chxq_conv_geom& g, PrepPla
     if (prep_rc != CHXQ_OK) return prep_rc;
     const int64_t rows = (int64_t)g.N * g.Ho * g.Wo;
     TcProblem p{};
-    p.a = a.x_out; p.C = a.cs; p.a_cs = a.cs;
+    if (a.pos_tiles > 0) {
+        p.a = a.x_out; p.C = a.cs; p.a_cs = a.cs;
+    } else {
+        p.a = x; p.C = g.C; p.a_cs = a.x_cs;
+    }
     const bool flat = P.pl.Wb == 128;  // a 1x1 convolution over the flattened map
     if (flat) {
         p.W = (int)rows; p.H = 1; p.N = 1;
@@ -1211,6 +1218,15 @@ int conv_dispatch(
     }
     const TcConvPlan pl = plan_tc_conv(*g);
     const bool aligned = (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
+    // NHWC: the map as it is, or, for a zero point that pads or weight zero points, the copy with border and pixel sums in place of an
+    // im2col matrix and a pass over every window; either way one launch in front of the kernel, where packing took three.
+    // One B200: [4, 64, 19, 19] 3 x 3 37 -> 8.8 us, [256, 128, 28, 28] 3 x 3 49 -> 43 us, with a zero point of 9 177 -> 53 us.
+    if (path != CHXQ_PATH_SIMT && g->group == 1 && pl.path == kTcDirect && aligned && g->x_layout == CHXQ_NHWC) {
+        const bool padded = g->pad_top || g->pad_left || g->pad_bottom || g->pad_right;
+        if (prep_plan(*g, epi.mode == kEpiInt32 ? 4 : 1, xz != 0, zw.len != 0, &pp, (padded && xz != 0) || zw.len != 0) && workspace != nullptr &&
+            workspace_bytes >= pp.total && (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0)
+            return conv_prep_run(x, w, *g, pp, xz, nullptr, zw, epi, y, static_cast<uint8_t*>(workspace), s);
+    }
     bool use_tc = path != CHXQ_PATH_SIMT && pl.path != kTcNone && aligned;
     if (g->group > 1 && use_tc) {
         // the grouped tensor-core path covers uint8 round-half-up epilogues (and raw accumulators) with absent weight zero points
@@ -1473,7 +1489,9 @@ extern "C" size_t chxq_conv_workspace(const chxq_conv_geom* g) {
     // Worst case over zero points: an explicit im2col matrix when the direct path cannot express the
     // padding value, and per-position sums when the weight zero point is non-zero.
     const size_t im2col = (pl.path == kTcIm2col || pl.path == kTcS2d || padded) ? L.im2col_bytes : 0;
-    return L.pack_total + im2col + L.rowsum_bytes;
+    const size_t general = L.pack_total + im2col + L.rowsum_bytes;
+    const size_t prep = pl.path == kTcDirect && g->group == 1 ? prep_workspace(*g) : 0;
+    return prep > general ? prep : general;
 }
 
 extern "C" size_t chxq_conv_packed_workspace(const chxq_conv_geom* g, int32_t x_zero_point, int32_t packed_flags) {

@@ -56,6 +56,7 @@ CONVS = [
     (1, 65, 12, 43, 70, 5, 1, 2),    # second channel tile of one channel, four positions that cross rows of the padded map
     (2, 130, 7, 7, 257, 3, 1, 1),    # several channel shares of the pixel sums
     (1, 16, 23, 23, 16, 1, 2, 0),    # strided 1x1
+    (2, 48, 10, 9, 24, 3, 2, 1),     # NHWC rows the tensor-core kernel reads as they are
     (2, 20, 6, 6, 40, 3, 1, 4),      # padding wider than the kernel
 ]
 
