@@ -481,6 +481,9 @@ __global__ void __launch_bounds__(kLinThreads, 1) linear_f32_kernel(
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
+    // Threads whose rows do not exist only copy: with one row, three of the four warps would read shared memory for nothing, which the
+    // fourth then waits for.  [1, 2048] x [1000, 2048]^T from cold caches: 16.8 -> 14.8 us.
+    const bool has_rows = n0 + tn * RN < N;
     float acc[RN][RO] = {};
 #pragma unroll
     for (int i = 0; i < T::kStages - 1; ++i) fetch(i, i);
@@ -493,6 +496,7 @@ __global__ void __launch_bounds__(kLinThreads, 1) linear_f32_kernel(
         const uint32_t st = smem0 + (uint32_t)(stage * T::kRows * T::kPitch * 4);
         const uint32_t xs = st + (uint32_t)(tn * RN * T::kPitch * 4), ws = st + (uint32_t)((T::kN + to) * T::kPitch * 4);
         stage = stage + 1 == T::kStages ? 0 : stage + 1;
+        if (!has_rows) continue;
         float4 xv[T::kDepth][RN], wv[T::kDepth][RO];
         auto load = [&](int buf, int k4) {
 #pragma unroll
