@@ -289,7 +289,11 @@ struct OwnScratch {
     at::Tensor t;
     void* get(size_t nbytes, const at::Tensor& like) {
         if (nbytes == 0) return nullptr;
-        t = at::detail::empty_cuda({(int64_t)nbytes}, at::kByte, like.device(), std::nullopt);
+        try {
+            t = at::detail::empty_cuda({(int64_t)nbytes}, at::kByte, like.device(), std::nullopt);
+        } catch (const c10::OutOfMemoryError&) {
+            return nullptr;  // the library then takes its form without scratch
+        }
         return t.data_ptr();
     }
 };
@@ -640,7 +644,7 @@ PyObject* conv_integer(PyObject*, Args a, Py_ssize_t n) {
         if (zx.scalar_type() != x.scalar_type()) fail(CHXQ_ERR_INVALID_ARGUMENT, "ConvInteger: a device x_zero_point must have x's dtype");
         const ZpArray zw = zp_array(a[3], w, "w_zero_point");
         OwnScratch own;
-        const size_t ws_bytes = chxq_conv_dev_workspace(&g);
+        const size_t ws_bytes = (int)as_long(a[8]) != CHXQ_PATH_SIMT ? chxq_conv_dev_workspace(&g) : 0;
         void* ws = own.get(ws_bytes, x);
         call([&] { return chxq_conv_integer_dev_ws(x.data_ptr(), w.data_ptr(), &g, zx.data_ptr(), zw.ptr, zw.len, yp, ws, ws_bytes, stream()); });
         return wrap(std::move(y));
