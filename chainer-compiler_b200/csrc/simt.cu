@@ -444,8 +444,6 @@ __global__ void __launch_bounds__(kLinThreads, 1) linear_f32_kernel(
         const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ b, int N, int K, int O, float* __restrict__ y) {
     constexpr int RN = T::RN, RO = T::RO;
     extern __shared__ __align__(16) float lin_smem[];  // [stage][kN rows of x, kO rows of w][pitch]
-    pdl_launch_dependents();
-    pdl_dependency_wait();
     const int tid = threadIdx.x;
     const int tn = tid / T::TO, to = tid % T::TO;
     const int n0 = blockIdx.y * T::kN, o0 = blockIdx.x * T::kO;
@@ -551,7 +549,10 @@ cudaError_t launch_linear(const float* x, const float* w, const float* b, int N,
         }
     }
     const dim3 grid((O + T::kO - 1) / T::kO, (N + T::kN - 1) / T::kN);
-    return launch_pdl(linear_f32_kernel<T>, grid, kLinThreads, T::kSmem, s, x, w, b, N, K, O, y);
+    // A plain launch: started early (programmatic dependent launch), the blocks fill the SMs that are idle then, two on each, and those
+    // finish last ([256, 2048] x [1000, 2048]^T: 78 us instead of 46).
+    linear_f32_kernel<T><<<grid, kLinThreads, T::kSmem, s>>>(x, w, b, N, K, O, y);
+    return cudaGetLastError();
 }
 
 // NCHW <-> NHWC transposes through a 32x32 shared tile over the (C, H*W) plane.
