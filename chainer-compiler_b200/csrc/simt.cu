@@ -550,7 +550,7 @@ cudaError_t launch_linear(const float* x, const float* w, const float* b, int N,
     }
     const dim3 grid((O + T::kO - 1) / T::kO, (N + T::kN - 1) / T::kN);
     // A plain launch: started early (programmatic dependent launch), the blocks fill the SMs that are idle then, two on each, and those
-    // finish last ([256, 2048] x [1000, 2048]^T: 78 us instead of 46).
+    // finish last ([256, 2048] x [1000, 2048]^T: 78 us instead of 49, call after call).
     linear_f32_kernel<T><<<grid, kLinThreads, T::kSmem, s>>>(x, w, b, N, K, O, y);
     return cudaGetLastError();
 }
