@@ -312,12 +312,13 @@ struct ZeroEntry {
 };
 
 bool weight_zero_points_are_zero(const at::Tensor& wz) {
+    if (wz.is_inference()) return false;  // no version counter, so nothing learned about it can be kept: the general form
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing((cudaStream_t)stream(), &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
         return false;  // no synchronization during a capture: the general form
     static auto& cache = *new std::map<std::tuple<const void*, int64_t, int>, ZeroEntry>;
     const auto key = std::make_tuple((const void*)wz.data_ptr(), wz.numel(), (int)wz.scalar_type());
-    const uint32_t version = wz.is_inference() ? 0u : wz._version();
+    const uint32_t version = wz._version();
     const auto it = cache.find(key);
     if (it != cache.end() && it->second.version == version && it->second.storage.lock().get() == wz.storage().unsafeGetStorageImpl()) return it->second.zero;
     const bool zero = !wz.ne(0).any().item<bool>();

@@ -1,0 +1,62 @@
+"""What the host bodies of the ops keep, hold and share: the answer about a weight zero point, the interpreter lock, errors raised inside a call,
+scratch on several streams."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _t(a, dev):
+    return torch.from_numpy(np.array(a)).to(dev)
+
+
+def _conv_case(ops, orc, dev, seed=0):
+    """(call(w_zero_point tensor), want(zero points)) of a small QLinearConv."""
+    rng = np.random.default_rng(seed)
+    x, w = rng.integers(0, 256, (2, 24, 9, 10), dtype=np.uint8), rng.integers(-127, 128, (16, 24, 3, 3)).astype(np.int8)
+    ws = rng.uniform(0.001, 0.002, 16).astype(np.float32)
+    xt, wt, wst = _t(x, dev), _t(w, dev), _t(ws, dev)
+
+    def call(wz):
+        return ops.QLinearConv(xt, 0.02, np.uint8(5), wt, wst, wz, 0.05, np.uint8(100), strides=(1, 1), pads=(1, 1)).cpu().numpy()
+
+    def want(wz):
+        return orc.requantize(orc.conv_integer(x, w, 5, wz, (1, 1), (1, 1)), 0.02, ws, 0.05, 100, channel_axis=1)
+
+    return call, want
+
+
+def test_weight_zero_points_changed_in_place(ops, orc, dev):
+    """A zero-point tensor that was all zeros and is changed in place: ordinary tensors, and inference tensors, which have no version counter."""
+    call, want = _conv_case(ops, orc, dev)
+    zero, other = want(np.zeros(16, np.int8)), want(np.full(16, 3, np.int8))
+    assert (zero != other).any()
+    for inference in (False, True):
+        with torch.inference_mode(inference):
+            wz = torch.zeros(16, dtype=torch.int8, device=dev)
+            assert wz.is_inference() == inference
+            assert np.array_equal(call(wz), zero)
+            wz.fill_(3)
+            assert np.array_equal(call(wz), other)
+            wz.zero_()
+            assert np.array_equal(call(wz), zero)
+    # an ordinary tensor changed under inference mode
+    wz = torch.zeros(16, dtype=torch.int8, device=dev)
+    assert np.array_equal(call(wz), zero)
+    with torch.inference_mode():
+        wz.fill_(3)
+        assert np.array_equal(call(wz), other)
+
+
+def test_weight_zero_points_at_a_reused_address(ops, orc, dev):
+    """What was learned about a tensor is not believed of the next one at its address."""
+    call, want = _conv_case(ops, orc, dev)
+    zero, other = want(np.zeros(16, np.int8)), want(np.full(16, 3, np.int8))
+    addresses = []
+    for value, expect in ((0, zero), (3, other), (0, zero)):
+        wz = torch.full((16,), value, dtype=torch.int8, device=dev)
+        addresses.append(wz.data_ptr())
+        assert np.array_equal(call(wz), expect)
+        del wz
+    assert len(set(addresses)) < 3  # the allocator did hand the block out again
