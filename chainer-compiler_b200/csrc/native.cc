@@ -58,14 +58,22 @@ PyObject* raise(const OpError& e) {
     return nullptr;
 }
 
+// The interpreter lock, given up until the end of the scope -- also by an exception (a tensor without storage throws when it is asked for its
+// address), which is turned into a Python one by code that needs the lock.
+struct Unlocked {
+    PyThreadState* save = PyEval_SaveThread();
+    Unlocked() = default;
+    Unlocked(const Unlocked&) = delete;
+    ~Unlocked() { PyEval_RestoreThread(save); }
+};
+
 // Runs a library call without the interpreter lock and turns its status into an exception.
 template <typename F>
 void call(F&& f) {
     int rc;
     {
-        PyThreadState* save = PyEval_SaveThread();
+        const Unlocked unlocked;
         rc = f();
-        PyEval_RestoreThread(save);
     }
     if (rc != CHXQ_OK) throw OpError{rc, chxq_last_error()};
 }

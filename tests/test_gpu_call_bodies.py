@@ -60,3 +60,12 @@ def test_weight_zero_points_at_a_reused_address(ops, orc, dev):
         assert np.array_equal(call(wz), expect)
         del wz
     assert len(set(addresses)) < 3  # the allocator did hand the block out again
+
+
+def test_error_inside_a_call_is_raised(ops, dev):
+    """A tensor without storage (here: a batched one) throws when the body asks for its address, at a point where the interpreter lock is given up."""
+    x = torch.rand((4, 8), device=dev)
+    for _ in range(2):
+        with pytest.raises(RuntimeError):
+            torch.vmap(lambda t: ops.QuantizeLinear(t, 0.1))(x)
+    assert ops.QuantizeLinear(x, 1.0).shape == x.shape
