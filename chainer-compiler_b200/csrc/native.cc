@@ -260,49 +260,24 @@ ZpArray zp_array(PyObject* o, const at::Tensor& like, const char* what) {
 
 // ---- scratch --------------------------------------------------------------------------------------------------------------
 
-// Grow-only scratch buffer per device.  A CUDA graph captured around these ops bakes the buffer's address into its kernel nodes; when a
-// later call needs more scratch a larger buffer is allocated and the superseded one is kept (a graph captured earlier goes on writing
-// its im2col data and row sums into memory that still belongs here, not into a block the allocator may have given to a live tensor).
-// Growth is geometric (at least 1.5x), so the kept buffers sum to less than three times the largest request.  Guarded by the
-// interpreter lock; the tensors are never destroyed (the process may end after the CUDA context does).
-struct Scratch {
-    std::map<int, at::Tensor> current;
-    std::vector<at::Tensor> retired;
-};
-Scratch& scratch_store() {
-    static Scratch* s = new Scratch;
-    return *s;
-}
-
-const at::Tensor& scratch_tensor(size_t nbytes, c10::Device device) {
-    const int idx = device.has_index() ? device.index() : c10::cuda::current_device();
-    at::Tensor& ws = scratch_store().current[idx];
-    if (!ws.defined() || (size_t)ws.numel() < nbytes) {
-        if (ws.defined()) {
-            scratch_store().retired.push_back(ws);
-            nbytes = std::max(nbytes, (size_t)(ws.numel() + ws.numel() / 2));
-        }
-        ws = at::detail::empty_cuda({(int64_t)nbytes}, at::kByte, c10::Device(c10::kCUDA, (c10::DeviceIndex)idx), std::nullopt);
-    }
-    return ws;
-}
-
-void* scratch(size_t nbytes, const at::Tensor& like) {
-    return nbytes == 0 ? nullptr : scratch_tensor(nbytes, like.device()).data_ptr();
-}
-
-// Scratch of one call, from the caching allocator on the call's stream: calls on several streams or threads stay independent of one another.
-// (The shared buffer orders nothing between streams.)
+// Scratch of one call, from the caching allocator on the device and stream the launch goes to: calls on several streams or threads stay
+// independent of one another, a graph captured around a call owns its scratch with the rest of its pool, and the block is reused by whatever
+// comes next on the stream.  (One grow-only buffer per device, as these bodies had, saves the allocator's half microsecond and lets two streams
+// overwrite each other's operands.)
 struct OwnScratch {
     at::Tensor t;
-    void* get(size_t nbytes, const at::Tensor& like) {
+    void* get(size_t nbytes) {
         if (nbytes == 0) return nullptr;
-        try {
-            t = at::detail::empty_cuda({(int64_t)nbytes}, at::kByte, like.device(), std::nullopt);
-        } catch (const c10::OutOfMemoryError&) {
-            return nullptr;  // the library then takes its form without scratch
-        }
+        t = at::detail::empty_cuda({(int64_t)nbytes}, at::kByte, c10::Device(c10::kCUDA, c10::cuda::current_device()), std::nullopt);
         return t.data_ptr();
+    }
+    // For calls that have a form without scratch, which the library takes when it gets none.
+    void* get_if_room(size_t nbytes) {
+        try {
+            return get(nbytes);
+        } catch (const c10::OutOfMemoryError&) {
+            return nullptr;
+        }
     }
 };
 
@@ -600,7 +575,7 @@ PyObject* matmul_integer(PyObject*, Args a, Py_ssize_t n) {
     at::Tensor y = empty_map(size, at::kInt, l, false);
     const size_t ws_bytes = path != CHXQ_PATH_SIMT ? chxq_matmul_integer_workspace(batch, M, N, K) : 0;
     OwnScratch own;
-    void* ws = K % 16 != 0 ? own.get(ws_bytes, l) : scratch(ws_bytes, l);
+    void* ws = K % 16 != 0 ? own.get_if_room(ws_bytes) : own.get(ws_bytes);
     call([&] {
         return chxq_matmul_integer(l.data_ptr(), cl, r.data_ptr(), cr, batch, M, N, K, za.ptr, za.len, zb.ptr, zb.len, static_cast<int32_t*>(y.data_ptr()), ws,
                                    ws_bytes, path, stream());
@@ -627,7 +602,7 @@ PyObject* qlinear_matmul(PyObject*, Args a, Py_ssize_t n) {
     at::Tensor y = empty_map({M, N}, qtype(zy.code), l, false);
     const size_t ws_bytes = path != CHXQ_PATH_SIMT ? chxq_matmul_integer_workspace(1, M, N, K) : 0;
     OwnScratch own;
-    void* ws = K % 16 != 0 ? own.get(ws_bytes, l) : scratch(ws_bytes, l);
+    void* ws = K % 16 != 0 ? own.get_if_room(ws_bytes) : own.get(ws_bytes);
     call([&] {
         return chxq_qlinear_matmul(l.data_ptr(), cl, sa, za.value, r.data_ptr(), cr, sb, zb.value, sy, zy.value, zy.code, M, N, K, mode, y.data_ptr(), ws,
                                    ws_bytes, path, stream());
@@ -654,7 +629,7 @@ PyObject* conv_integer(PyObject*, Args a, Py_ssize_t n) {
         const ZpArray zw = zp_array(a[3], w, "w_zero_point");
         OwnScratch own;
         const size_t ws_bytes = (int)as_long(a[8]) != CHXQ_PATH_SIMT ? chxq_conv_dev_workspace(&g) : 0;
-        void* ws = own.get(ws_bytes, x);
+        void* ws = own.get_if_room(ws_bytes);
         call([&] { return chxq_conv_integer_dev_ws(x.data_ptr(), w.data_ptr(), &g, zx.data_ptr(), zw.ptr, zw.len, yp, ws, ws_bytes, stream()); });
         return wrap(std::move(y));
     }
@@ -662,7 +637,8 @@ PyObject* conv_integer(PyObject*, Args a, Py_ssize_t n) {
     const ZpArray zw = zp_array(a[3], w, "w_zero_point");
     const int path = (int)as_long(a[8]);
     const size_t ws_bytes = path != CHXQ_PATH_SIMT ? chxq_conv_workspace(&g) : 0;
-    void* ws = scratch(ws_bytes, x);
+    OwnScratch own;
+    void* ws = own.get(ws_bytes);
     call([&] {
         return chxq_conv_integer(x.data_ptr(), w.data_ptr(), &g, a[2] != Py_None, zx.value, zw.ptr, zw.len, yp, ws, ws_bytes, path, stream());
     });
@@ -691,7 +667,8 @@ PyObject* qlinear_conv(PyObject*, Args a, Py_ssize_t n) {
     w = w.contiguous();
     const int path = (int)as_long(a[6]);
     const size_t ws_bytes = path != CHXQ_PATH_SIMT ? chxq_conv_workspace(&g) : 0;
-    void* ws = scratch(ws_bytes, x);
+    OwnScratch own;
+    void* ws = own.get(ws_bytes);
     call([&] { return chxq_qlinear_conv(x.data_ptr(), w.data_ptr(), &g, &p.p, y.data_ptr(), ws, ws_bytes, path, stream()); });
     return wrap(std::move(y));
     OP_END
@@ -714,7 +691,8 @@ PyObject* qlinear_conv_packed(PyObject*, Args a, Py_ssize_t n) {
     at::Tensor y = output_map("QLinearConvPacked", a[2], size, qtype(p.y_code), x);
     if (!eligible(k)) fail(CHXQ_ERR_UNSUPPORTED, "QLinearConvPacked: this geometry is not eligible for the packed tensor-core path");
     const size_t ws_bytes = chxq_conv_packed_workspace(&g, p.p.x_zero_point, k.flags);
-    void* ws = scratch(ws_bytes, x);
+    OwnScratch own;
+    void* ws = own.get(ws_bytes);
     call([&] { return chxq_qlinear_conv_packed(x.data_ptr(), k.blob.data_ptr(), &g, &p.p, k.flags, y.data_ptr(), ws, ws_bytes, stream()); });
     return wrap(std::move(y));
     OP_END
@@ -775,7 +753,8 @@ PyObject* qlinear_conv_maxpool_packed(PyObject*, Args a, Py_ssize_t n) {
     if (stride < 1) fail(CHXQ_ERR_UNSUPPORTED, "%s: bad pooling stride", op);
     at::Tensor y = a[7] != Py_None ? tensor(a[7], "out") : empty_map({g.N, g.M, pooled(g.Ho), pooled(g.Wo)}, at::kByte, x, true);
     const size_t ws_bytes = chxq_conv_packed_workspace(&g, p.p.x_zero_point, k.flags);
-    void* ws = scratch(ws_bytes, x);
+    OwnScratch own;
+    void* ws = own.get(ws_bytes);
     call([&] {
         return chxq_qlinear_conv_maxpool_packed(x.data_ptr(), f32, mode, k.blob.data_ptr(), &g, &p.p, k.flags, (int)kernel, (int)stride, (int)pad, cover_all,
                                                 y.data_ptr(), ws, ws_bytes, stream());
@@ -801,7 +780,8 @@ PyObject* quantize_qlinear_conv_packed(PyObject*, Args a, Py_ssize_t n) {
     at::Tensor y = a[3] != Py_None ? tensor(a[3], "out") : empty_map({g.N, g.M, g.Ho, g.Wo}, qtype(p.y_code), x, true);
     if (!eligible(k)) fail(CHXQ_ERR_UNSUPPORTED, "%s: this geometry is not eligible for the packed tensor-core path", op);
     const size_t ws_bytes = chxq_conv_packed_workspace(&g, p.p.x_zero_point, k.flags);
-    void* ws = scratch(ws_bytes, x);
+    OwnScratch own;
+    void* ws = own.get(ws_bytes);
     call([&] {
         return chxq_quantize_qlinear_conv_packed(static_cast<const float*>(x.data_ptr()), mode, k.blob.data_ptr(), &g, &p.p, k.flags, y.data_ptr(), ws, ws_bytes,
                                                  stream());
@@ -823,7 +803,8 @@ PyObject* conv_integer_packed(PyObject*, Args a, Py_ssize_t n) {
     const Zp zx = zp_scalar(a[2]);
     at::Tensor y = empty_map({g.N, g.M, g.Ho, g.Wo}, at::kInt, x, true);
     const size_t ws_bytes = chxq_conv_packed_workspace(&g, zx.value, k.flags);
-    void* ws = scratch(ws_bytes, x);
+    OwnScratch own;
+    void* ws = own.get(ws_bytes);
     call([&] {
         return chxq_conv_integer_packed(x.data_ptr(), k.blob.data_ptr(), &g, a[2] != Py_None, zx.value, k.flags, static_cast<int32_t*>(y.data_ptr()), ws, ws_bytes,
                                         stream());
@@ -1035,16 +1016,6 @@ PyObject* transpose_map(PyObject*, Args a, Py_ssize_t n) {
     OP_END
 }
 
-// nbytes, device index (-1: current)
-PyObject* workspace(PyObject*, Args a, Py_ssize_t n) {
-    OP_BEGIN
-    need_args("workspace", n, 2);
-    const int idx = (int)as_long(a[1]);
-    at::Tensor t = scratch_tensor((size_t)as_long(a[0]), c10::Device(c10::kCUDA, (c10::DeviceIndex)idx));
-    return wrap(std::move(t));
-    OP_END
-}
-
 // ChxqError, ops._zp_scalar, ops._to_device_array, numpy.uint8, numpy.int8
 PyObject* setup(PyObject*, Args a, Py_ssize_t n) {
     OP_BEGIN
@@ -1063,7 +1034,7 @@ PyObject* setup(PyObject*, Args a, Py_ssize_t n) {
 PyMethodDef g_methods[] = {FAST(quantize_linear), FAST(dequantize_linear), FAST(matmul_integer), FAST(qlinear_matmul), FAST(conv_integer), FAST(qlinear_conv),
                            FAST(qlinear_conv_packed), FAST(qlinear_conv_chain_packed), FAST(qlinear_conv_maxpool_packed), FAST(quantize_qlinear_conv_packed),
                            FAST(conv_integer_packed), FAST(elementwise), FAST(maxpool_u8), FAST(global_avgpool_dq), FAST(linear), FAST(qadd_u8),
-                           FAST(dynamic_params_u8), {"minmax", minmax, METH_O, nullptr}, FAST(transpose_map), FAST(workspace), FAST(setup),
+                           FAST(dynamic_params_u8), {"minmax", minmax, METH_O, nullptr}, FAST(transpose_map), FAST(setup),
                            {nullptr, nullptr, 0, nullptr}};
 PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_native", "Host bodies of the VM ops over the C ABI of libchxq.so.", -1, g_methods, nullptr, nullptr, nullptr, nullptr};
 

@@ -54,12 +54,9 @@ def _qcode(t, what):
 
 
 def workspace(nbytes, device):
-    """Grow-only scratch buffer per device, 256-byte aligned (the op body owns scratch, as it owns outputs).  Superseded buffers are
-    kept, because captured CUDA graphs hold their raw addresses; growth is geometric."""
-    if nbytes == 0:
-        return None
-    device = torch.device(device)
-    return _native.workspace(int(nbytes), device.index if device.index is not None else torch.cuda.current_device())
+    """Scratch for one library call on the current stream, 256-byte aligned: a block of the caching allocator, the caller's until it lets
+    go of the tensor.  (Calls on other streams and in other threads have their own.)"""
+    return None if nbytes == 0 else torch.empty(int(nbytes), dtype=torch.uint8, device=device)
 
 
 def _to_device_array(v, like, kind):

@@ -69,3 +69,38 @@ def test_error_inside_a_call_is_raised(ops, dev):
         with pytest.raises(RuntimeError):
             torch.vmap(lambda t: ops.QuantizeLinear(t, 0.1))(x)
     assert ops.QuantizeLinear(x, 1.0).shape == x.shape
+
+
+def test_scratch_of_two_streams(ops, orc, dev):
+    """Calls that fill scratch (repacked operands, column terms, NHWC copies, packed weights, stem blocks), overlapping on two streams with operands of
+    their own: the results of the calls one after the other."""
+    gen = torch.Generator(device=dev).manual_seed(7)
+    u8 = lambda *s: torch.randint(0, 256, s, dtype=torch.uint8, device=dev, generator=gen)  # noqa: E731
+    s8 = lambda *s: torch.randint(-127, 128, s, dtype=torch.int8, device=dev, generator=gen)  # noqa: E731
+    z = torch.tensor([9], dtype=torch.uint8, device=dev)
+
+    def problem():
+        a, b, x, w, xs, wst = u8(256, 2048), s8(2048, 2048), u8(4, 128, 28, 28), s8(128, 128, 3, 3), u8(8, 3, 112, 112), s8(64, 3, 7, 7)
+        ws, wz = torch.rand(128, device=dev, generator=gen) * 1e-3 + 1e-3, torch.full((128,), 3, dtype=torch.int8, device=dev)
+        pk = ops.PackedConv(wst, wz[:64] * 0, xs.shape, (2, 2), (3, 3), x_layout=ops.NCHW)
+        return [lambda: ops.MatMulInteger(a, b, z, None),
+                lambda: ops.QLinearMatMul(a, 0.01, np.uint8(9), b, 0.01, np.int8(0), 30.0, np.uint8(9)),
+                lambda: ops.ConvInteger(x, w, np.uint8(9), None, (1, 1), (1, 1)),
+                lambda: ops.QLinearConv(x, 0.02, np.uint8(9), w, ws, wz, 0.5, np.uint8(99), strides=(1, 1), pads=(1, 1)),
+                lambda: ops.ConvIntegerPacked(xs, pk, np.uint8(3))]
+
+    problems = [problem(), problem()]
+    want = [[f() for f in p] for p in problems]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    got = [[], []]
+    for _ in range(8):
+        for i in range(len(problems[0])):
+            for k in range(2):
+                with torch.cuda.stream(streams[k]):
+                    got[k].append((i, problems[k][i]()))
+    torch.cuda.synchronize()
+    for k in range(2):
+        for i, y in got[k]:
+            assert torch.equal(y, want[k][i]), (k, i)
+    ops.device_status()
