@@ -304,7 +304,11 @@ bool weight_zero_points_are_zero(const at::Tensor& wz) {
     const uint32_t version = wz._version();
     const auto it = cache.find(key);
     if (it != cache.end() && it->second.version == version && it->second.storage.lock().get() == wz.storage().unsafeGetStorageImpl()) return it->second.zero;
-    const bool zero = !wz.ne(0).any().item<bool>();
+    bool zero;
+    {
+        const Unlocked unlocked;  // the read waits for the stream: other Python threads go on meanwhile
+        zero = !wz.ne(0).any().item<bool>();
+    }
     if (cache.size() > 4096) cache.clear();
     cache.insert_or_assign(key, ZeroEntry{c10::weak_intrusive_ptr<c10::StorageImpl>(wz.storage().getWeakStorageImpl()), version, zero});
     return zero;

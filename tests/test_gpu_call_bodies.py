@@ -1,5 +1,8 @@
 """What the host bodies of the ops keep, hold and share: the answer about a weight zero point, the interpreter lock, errors raised inside a call,
 scratch on several streams."""
+import threading
+import time
+
 import numpy as np
 import pytest
 import torch
@@ -104,3 +107,28 @@ def test_scratch_of_two_streams(ops, orc, dev):
         for i, y in got[k]:
             assert torch.equal(y, want[k][i]), (k, i)
     ops.device_status()
+
+
+def test_other_threads_run_while_a_zero_point_is_read(ops, orc, dev):
+    """A weight zero point that the body has not seen is read from the device, behind whatever the stream has queued: that wait must not keep other
+    Python threads from running."""
+    call, want = _conv_case(ops, orc, dev)
+    expect = want(np.zeros(16, np.int8))
+    fresh = [torch.zeros(16, dtype=torch.int8, device=dev) for _ in range(2)]
+    call(fresh[0])  # everything loaded
+    done = []
+
+    def body():
+        torch.cuda._sleep(1_000_000_000)  # about half a second of this thread's stream
+        done.append(call(fresh[1]))
+
+    thread = threading.Thread(target=body)
+    worst, last = 0.0, time.perf_counter()
+    thread.start()
+    while thread.is_alive():
+        time.sleep(0.001)
+        now = time.perf_counter()
+        worst, last = max(worst, now - last), now
+    thread.join()
+    assert np.array_equal(done[0], expect)
+    assert worst < 0.2, "the main thread stood still for %.2f s" % worst
