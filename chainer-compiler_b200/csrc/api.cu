@@ -1247,8 +1247,10 @@ int conv_dispatch(
     if (path != CHXQ_PATH_SIMT && g->group == 1 && pl.path == kTcDirect && aligned && g->x_layout == CHXQ_NHWC) {
         const bool padded = g->pad_top || g->pad_left || g->pad_bottom || g->pad_right;
         if (prep_plan(*g, epi.mode == kEpiInt32 ? 4 : 1, xz != 0, zw.len != 0, &pp, (padded && xz != 0) || zw.len != 0) && workspace != nullptr &&
-            workspace_bytes >= pp.total && (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0)
-            return conv_prep_run(x, w, *g, pp, xz, nullptr, zw, epi, y, static_cast<uint8_t*>(workspace), s);
+            workspace_bytes >= pp.total && (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0) {
+            rc = conv_prep_run(x, w, *g, pp, xz, nullptr, zw, epi, y, static_cast<uint8_t*>(workspace), s);
+            if (!(rc == CHXQ_ERR_UNSUPPORTED && path == CHXQ_PATH_AUTO)) return rc;  // else the forms below
+        }
     }
     bool use_tc = path != CHXQ_PATH_SIMT && pl.path != kTcNone && aligned;
     if (g->group > 1 && use_tc) {

@@ -2,6 +2,7 @@
 // tc_bk32.cu / tc_bk64.cu / tc_bk128.cu): planning of tile shapes, tensor maps, dispatch and optional per-launch timing.
 #include <cuda.h>
 
+#include <algorithm>
 #include <atomic>
 #include <mutex>
 #include <vector>
@@ -133,13 +134,14 @@ static void choose_tile(const chxq_conv_geom& g, TcConvPlan* pl) {
     auto tiles = [&](int wb, int hb, int nb) {
         return (int64_t)((g.Wo + wb - 1) / wb) * ((g.Ho + hb - 1) / hb) * ((g.N + nb - 1) / nb);
     };
+    const int max_rows = 256 / g.stride_h;  // extent of a TMA box, in output rows
     pl->Wb = largest_pow2_divisor(g.Wo, 16);
-    pl->Hb = largest_pow2_divisor(g.Ho, 128 / pl->Wb);
+    pl->Hb = largest_pow2_divisor(g.Ho, std::min(128 / pl->Wb, max_rows));
     pl->Nb = 128 / (pl->Wb * pl->Hb);
     int64_t best = tiles(pl->Wb, pl->Hb, pl->Nb);
     for (int wb = 16; wb >= 1; wb /= 2)
         for (int hb = 128 / wb; hb >= 1; hb /= 2) {
-            if (hb * g.stride_h > 256) continue;  // extent of a TMA box
+            if (hb > max_rows) continue;
             const int64_t t = tiles(wb, hb, 128 / (wb * hb));
             if (t < best) {
                 best = t;

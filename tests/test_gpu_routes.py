@@ -124,3 +124,19 @@ def test_small_batch_split_k(ops, pkg, orc, dev, N, C, H, W, M, k, s):
             finally:
                 pkg.lib().chxq_tc_variant(0)
         assert np.array_equal(got[0], want) and np.array_equal(got[1], want)
+
+
+# the position box of a strided convolution has to fit a TMA box: 256 input rows
+@pytest.mark.parametrize("N,H,W,k,s,p", [(2, 382, 19, 3, (3, 3), (1, 1)), (2, 509, 1, 1, (4, 1), (0, 0)), (1, 1017, 3, 1, (8, 8), (0, 0))])
+def test_strided_conv_tall_box(ops, orc, dev, N, H, W, k, s, p):
+    rng = np.random.default_rng(H)
+    x, w = _rand(rng, (N, 16, H, W), np.uint8), _rand(rng, (8, 16, k, k), np.int8)
+    zw = _rand(rng, 8, np.int8)
+    wt, xt = _t(w, dev), _t(x, dev)
+    for zx in (0, 9):
+        for zp in (None, zw):
+            want = orc.conv_integer(x, w, zx, zp, s, p)
+            for xin in (xt, xt.contiguous(memory_format=torch.channels_last)):
+                for path in (ops.PATH_AUTO, ops.PATH_TENSOR):
+                    y = ops.ConvInteger(xin, wt, np.uint8(zx), None if zp is None else _t(zp, dev), s, p, path=path)
+                    assert np.array_equal(y.cpu().numpy(), want), (zx, zp is None, xin.stride(), path)
