@@ -1110,9 +1110,14 @@ bool prep_plan(const chxq_conv_geom& g, int y_elem, bool border, bool pixel_sums
     return true;
 }
 
-size_t prep_workspace(const chxq_conv_geom& g) {  // the largest over the forms a call may take
-    PrepPlan P;
-    return prep_plan(g, 1, true, true, &P) ? P.total : 0;
+// The largest over the forms a call may take, or 0 if one of them has no such plan.  Pixel sums only add to it; a map without border is smaller,
+// but may have its pixel sums in more shares.
+size_t prep_workspace(const chxq_conv_geom& g) {
+    PrepPlan P, Q;
+    if (!prep_plan(g, 1, true, true, &P)) return 0;
+    if (!P.prep.border) return P.total;
+    if (!prep_plan(g, 1, false, true, &Q)) return 0;
+    return P.total > Q.total ? P.total : Q.total;
 }
 
 int conv_prep_run(const void* x, const void* w, const chxq_conv_geom& g, PrepPlan& P, int x_zp, const void* x_zp_dev, const ZpSpec& zw,
@@ -1503,8 +1508,10 @@ extern "C" int chxq_conv_resolve_geometry(
 
 extern "C" size_t chxq_conv_workspace(const chxq_conv_geom* g) {
     if (!g || validate_geom("conv workspace", g) != CHXQ_OK) return 0;
-    PrepPlan pp;
-    if (g->C > 4 && g->x_layout == CHXQ_NCHW && g->y_layout == CHXQ_NCHW && g->N <= 65535 && prep_plan(*g, 1, true, true, &pp)) return pp.total;
+    if (g->C > 4 && g->x_layout == CHXQ_NCHW && g->y_layout == CHXQ_NCHW && g->N <= 65535) {
+        const size_t prep = prep_workspace(*g);
+        if (prep > 0) return prep;
+    }
     NchwPlan np;
     if (nchw_plan(*g, 4, &np)) return np.x_bytes + np.y_bytes + inner_conv_workspace(np.g2);  // sized for int32 outputs (ConvInteger), the larger case
     const TcConvPlan pl = plan_tc_conv(*g);

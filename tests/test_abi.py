@@ -202,3 +202,42 @@ def test_generated_source_compiles_for_sm100a(pkg, dtype):
              Node("Identity", ["y"], ["z"])]
     ok, log = _nvrtc_compile(build_program(nodes, 5, ["x"], ["z", "e"], dtype), "fusion5")
     assert ok, log
+
+
+def _workspace_needed(L, _lib, g, int32_out, x_zp, w_zp):
+    """Bytes the tensor-core form of an NCHW call asks for: a TENSOR call without workspace is refused with that number, before anything is
+    launched or read (the buffers here are never looked at)."""
+    any_ptr = ctypes.c_void_p(4096)
+    if int32_out:
+        rc = L.chxq_conv_integer(any_ptr, any_ptr, ctypes.byref(g), 1, x_zp, any_ptr if w_zp else None, w_zp, any_ptr, None, 0, _lib.PATH_TENSOR, None)
+    else:
+        p = _lib.QConvParams()
+        p.x_scale, p.x_zero_point, p.w_scale, p.w_zero_point, p.w_params_len = 0.1, x_zp, 4096, 4096 if w_zp else None, 1
+        p.y_scale, p.y_dtype, p.clamp_hi_q = 0.1, _lib.UINT8, -1
+        rc = L.chxq_qlinear_conv(any_ptr, any_ptr, ctypes.byref(g), ctypes.byref(p), any_ptr, None, 0, _lib.PATH_TENSOR, None)
+    assert rc == _lib.ERR_WORKSPACE, L.chxq_last_error()
+    return int(re.search(rb"needs (\d+) bytes", L.chxq_last_error()).group(1))
+
+
+def test_conv_workspace_covers_every_form(pkg):
+    """chxq_conv_workspace does not know the zero points: it has to be enough with and without them, for both output types."""
+    from chainer_compiler_b200 import _lib
+    L = pkg.lib()
+    rng = np.random.default_rng(11)
+    cases = [(6, 80, 112, 112, 16, 3, 3, 1, 1, 1), (148, 256, 128, 1, 256, 3, 1, 1, 0, 1), (78, 128, 128, 8, 64, 3, 1, 1, 0, 1), (7, 91, 103, 103, 8, 3, 3, 1, 1, 1)]
+    for _ in range(600):
+        n, c, h, w = (int(round(np.exp(rng.uniform(np.log(lo), np.log(hi))))) for lo, hi in ((1, 300), (5, 400), (1, 240), (1, 240)))
+        kh, kw = (int(k) for k in rng.choice([1, 2, 3, 5, 7], 2))
+        ph, pw = int(rng.integers(0, kh + 1)), int(rng.integers(0, kw + 1))
+        cases.append((n, c, h, w, int(rng.integers(1, 200)), kh, kw, ph, pw, int(rng.integers(1, 4))))
+    checked = 0
+    for n, c, h, w, m, kh, kw, ph, pw, s in cases:
+        if h + 2 * ph < kh or w + 2 * pw < kw:
+            continue
+        rc, g = _geom(pkg, n, c, h, w, m, c, kh, kw, (s, s), (ph, pw), 1, "")
+        assert rc == 0
+        for int32_out in (False, True):
+            need = max(_workspace_needed(L, _lib, g, int32_out, x_zp, w_zp) for x_zp in (0, 9) for w_zp in (0, 1))
+            assert L.chxq_conv_workspace(ctypes.byref(g)) >= need, (n, c, h, w, m, kh, kw, ph, pw, s)
+        checked += 1
+    assert checked > 400

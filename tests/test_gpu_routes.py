@@ -140,3 +140,17 @@ def test_strided_conv_tall_box(ops, orc, dev, N, H, W, k, s, p):
                 for path in (ops.PATH_AUTO, ops.PATH_TENSOR):
                     y = ops.ConvInteger(xin, wt, np.uint8(zx), None if zp is None else _t(zp, dev), s, p, path=path)
                     assert np.array_equal(y.cpu().numpy(), want), (zx, zp is None, xin.stride(), path)
+
+
+# no zero point of x, zero points of w: fewer position tiles than with a border, so more channel shares of the pixel sums
+@pytest.mark.parametrize("N,C,H,W,M,k,p", [(6, 80, 112, 112, 16, 3, 1), (78, 128, 128, 8, 64, 3, (1, 0))])
+def test_conv_pixel_sums_fit_the_reported_workspace(ops, dev, N, C, H, W, M, k, p):
+    gen = torch.Generator(device=dev).manual_seed(C)
+    kw = k if isinstance(p, int) else 1
+    pads = (p, p) if isinstance(p, int) else p
+    x = torch.randint(0, 256, (N, C, H, W), dtype=torch.uint8, device=dev, generator=gen)
+    w = torch.randint(-127, 128, (M, C, k, kw), dtype=torch.int8, device=dev, generator=gen)
+    zw = torch.randint(-9, 10, (M,), dtype=torch.int8, device=dev, generator=gen)
+    ws = torch.rand(M, device=dev, generator=gen) * 1e-3 + 1e-3
+    args = (x, 0.02, np.uint8(0), w, ws, zw, 0.9, np.uint8(100), None, (1, 1), pads)
+    assert torch.equal(ops.QLinearConv(*args, path=ops.PATH_TENSOR), ops.QLinearConv(*args, path=ops.PATH_SIMT))
