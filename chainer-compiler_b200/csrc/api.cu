@@ -744,11 +744,17 @@ bool gemm_tc_eligible(const void* a, int64_t M, int64_t N, int64_t K) {
            K < (1ll << 31);
 }
 
-// Rows of A that do not start on sixteen-byte boundaries (K % 16 != 0) reach the tensor cores through a copy at a wider pitch.  The copy
-// is one pass over A; the CUDA-core kernel makes one multiply-add per lane and clock.  One B200, whole calls: 509 x 3073 x 1283 with zero
-// points 293 -> 22 us, the 784-1000-1000-10 MLP of 64 rows (two of its three products have K = 1000) 104 -> 39 us.
-bool gemm_tc_via_copy(int64_t M, int64_t N, int64_t K) {
-    return K % 16 != 0 && K >= 16 && M >= 1 && N >= 1 && M < (1ll << 31) && N < (1ll << 31) && K < (1ll << 20);
+// Rows of A that do not start on sixteen-byte boundaries (K % 16 != 0) can reach the tensor cores through a copy at a wider pitch, in two
+// launches per matrix; the CUDA-core kernel takes the whole batch in one.  Which of them is estimated to finish first: the copy and the
+// product cost 7 us a matrix and a pass over both operands, the CUDA-core kernel 2 us, 27 steps of its K chain a microsecond and 7.3 million
+// multiply-adds a microsecond.  One B200, device time, copy / CUDA cores: 512 x [49 x 49 x 50] 3600 / 23 us, 8 x [512 x 512 x 500] 67 / 147 us,
+// 49 x 49 x 50 7.0 / 4.1 us, 128 x 128 x 250 7.0 / 12.4 us, 509 x 3073 x 1283 22 / 293 us; over 220 products of 1 to 64 matrices, extents up
+// to 3000, the choice costs 0.2 % on the geometric mean against the faster of the two (the copy alone 152 %, the CUDA cores alone 34 %).
+bool gemm_tc_via_copy(int64_t batch, int64_t M, int64_t N, int64_t K) {
+    if (K % 16 == 0 || K < 16 || M < 1 || N < 1 || M >= (1ll << 31) || N >= (1ll << 31) || K >= (1ll << 20)) return false;
+    const double copy_us = (double)batch * (7.0 + ((double)M + (double)N) * (double)K / 6e5);
+    const double simt_us = 2.0 + (double)K / 27.0 + (double)batch * (double)M * (double)N * (double)K / 7.3e6;
+    return copy_us < simt_us;
 }
 
 int gemm_dispatch(
@@ -757,7 +763,7 @@ int gemm_dispatch(
         cudaStream_t s) {
     if (batch == 0 || M == 0 || N == 0) return CHXQ_OK;
     const bool tc_ok = gemm_tc_eligible(a, M, N, K) && ((M * K) % 16 == 0 || batch == 1);
-    bool use_tc = path == CHXQ_PATH_TENSOR || (path == CHXQ_PATH_AUTO && (tc_ok || gemm_tc_via_copy(M, N, K)));
+    bool use_tc = path == CHXQ_PATH_TENSOR || (path == CHXQ_PATH_AUTO && (tc_ok || gemm_tc_via_copy(batch, M, N, K)));
     if (path == CHXQ_PATH_TENSOR && !tc_ok)
         return set_error(CHXQ_ERR_UNSUPPORTED, "%s: tensor-core path needs K %% 16 == 0 and a 16-byte aligned A (M=%lld N=%lld K=%lld)", op,
                          (long long)M, (long long)N, (long long)K);

@@ -154,3 +154,19 @@ def test_conv_pixel_sums_fit_the_reported_workspace(ops, dev, N, C, H, W, M, k, 
     ws = torch.rand(M, device=dev, generator=gen) * 1e-3 + 1e-3
     args = (x, 0.02, np.uint8(0), w, ws, zw, 0.9, np.uint8(100), None, (1, 1), pads)
     assert torch.equal(ops.QLinearConv(*args, path=ops.PATH_TENSOR), ops.QLinearConv(*args, path=ops.PATH_SIMT))
+
+
+# (batch, M, N, K, launches): the copy and the product (two launches a matrix) where they are faster than the one of the CUDA cores
+@pytest.mark.parametrize("batch,M,N,K,launches", [(1, 1, 1, 137, 2), (1, 7, 3, 145, 2), (1, 8, 63, 201, 2), (1, 9, 65, 255, 2), (1, 129, 64, 193, 2), (2, 5, 21, 401, 4),
+                                                  (3, 130, 257, 1283, 6), (1, 49, 49, 50, 1), (512, 49, 49, 50, 1), (5, 70, 33, 197, 1)])
+def test_matmul_ragged_k_launches(ops, pkg, orc, dev, batch, M, N, K, launches):
+    rng = np.random.default_rng(batch + M + N + K)
+    lead = () if batch == 1 else (batch,)
+    a, b = _rand(rng, lead + (M, K), np.uint8), _rand(rng, lead + (K, N), np.int8)
+    za, zb = _rand(rng, K, np.uint8), _rand(rng, N, np.int8)
+    at, bt = _t(a, dev), _t(b, dev)
+    for z0, z1 in ((None, None), (za[:1], zb), (za, zb[:1])):
+        before = pkg.lib().chxq_launch_count()
+        y = ops.MatMulInteger(at, bt, None if z0 is None else _t(z0, dev), None if z1 is None else _t(z1, dev))
+        assert pkg.lib().chxq_launch_count() - before == launches
+        assert np.array_equal(y.cpu().numpy(), orc.matmul_integer(a, b, z0, z1)), (z0 is None, z1 is None)
