@@ -1567,6 +1567,17 @@ extern "C" int chxq_conv_integer_dev(
     return launch_conv_simt(x, w, *g, 1, 0, w_zero_point, w_zp_len, epi, y, as_stream(stream), x_zero_point);
 }
 
+// ConvInteger with a device zero point: whether preparing and multiplying on the tensor cores (two launches) is estimated to finish before the
+// CUDA-core kernel (one).  Least-squares fits in microseconds over 260 convolutions of up to 16 images, 80 channels and 48 x 48 positions on
+// one B200; the choice costs 0.9 % on the geometric mean against the faster of the two (the tensor cores alone 24 %, the CUDA cores alone 38 %).
+// [1, 3, 7, 7] 3 x 3 to 16 channels 8.8 / 5.8 us, [1, 64, 7, 7] 3 x 3 to 64 9.8 / 35.5 us, [8, 64, 56, 56] 3 x 3 to 64 20 / 1180 us.
+static bool conv_dev_tc_pays(const chxq_conv_geom& g, bool w_zp) {
+    const double K = (double)g.C * g.KH * g.KW, outputs = (double)g.N * g.M * g.Ho * g.Wo;
+    const double tc_us = 5.3 + (g.KH * g.KW > 1 ? 3.1 : 0.0) + (w_zp ? 0.8 : 0.0) + (double)g.N * g.H * g.W * ((g.C + 15) / 16 * 16) * 8.4e-6;
+    const double simt_us = 3.4 + K / 20.0 + outputs * (K + 21.0) / 1.34e6;
+    return tc_us < simt_us;
+}
+
 extern "C" size_t chxq_conv_dev_workspace(const chxq_conv_geom* g) {
     if (!g || validate_geom("conv workspace", g) != CHXQ_OK) return 0;
     return prep_workspace(*g);
@@ -1577,8 +1588,8 @@ extern "C" int chxq_conv_integer_dev_ws(
         void* workspace, size_t workspace_bytes, void* stream) {
     PrepPlan pp;
     if (g != nullptr && validate_geom("ConvInteger", g) == CHXQ_OK && (int64_t)g->N * g->M * g->Ho * g->Wo != 0 && x && w && y && x_zero_point &&
-        check_zp_len("ConvInteger", "w_zero_point", w_zero_point, w_zp_len, g->M) == CHXQ_OK && prep_plan(*g, 4, true, w_zp_len != 0, &pp) &&
-        workspace != nullptr && workspace_bytes >= pp.total && (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0) {
+        check_zp_len("ConvInteger", "w_zero_point", w_zero_point, w_zp_len, g->M) == CHXQ_OK && conv_dev_tc_pays(*g, w_zp_len != 0) &&
+        prep_plan(*g, 4, true, w_zp_len != 0, &pp) && workspace != nullptr && workspace_bytes >= pp.total && (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0) {
         EpiArgs epi{};
         epi.mode = kEpiInt32;
         const int rc = conv_prep_run(x, w, *g, pp, 0, x_zero_point, ZpSpec{w_zero_point, w_zp_len, 0}, epi, y, static_cast<uint8_t*>(workspace), as_stream(stream));

@@ -155,7 +155,7 @@ def ConvInteger(x, w, x_zero_point=None, w_zero_point=None, strides=(), pads=(),
     """runtime/chxvm_defs.py:466-469; body runtime/ops/quantize.cc:116-146.
 
     x_zero_point may be a one-element CUDA tensor of x's dtype (a zero point computed on the device): it is then read by the
-    kernel, not by the host (on the tensor cores; grouped convolutions and PATH_SIMT on the general CUDA-core kernel)."""
+    kernel, not by the host (on the tensor cores; tiny and grouped convolutions and PATH_SIMT on the general CUDA-core kernel)."""
     return _native.conv_integer(x, w, x_zero_point, w_zero_point, strides, pads, group, auto_pad, path)
 
 

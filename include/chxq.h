@@ -359,8 +359,9 @@ int chxq_minmax_f32(const float* x, int64_t n, float* out2, void* stream);
  *     device memory; same element arithmetic (runtime/ops/quantize.cc:16-35).
  *   chxq_conv_integer_dev: chxq_conv_integer (runtime/ops/quantize.cc:116-146) with the activation zero point read from a device
  *     scalar of x's dtype; without scratch it runs on the general CUDA-core kernel.
- *   chxq_conv_integer_dev_ws: the same on the tensor cores, with chxq_conv_dev_workspace bytes of 256-byte aligned scratch; falls back to
- *     the general kernel where the geometry has no such form (groups, negative pads, strides above 8) or the scratch is too small.
+ *   chxq_conv_integer_dev_ws: the same, on the tensor cores where they are the faster of the two, with chxq_conv_dev_workspace bytes of 256-byte
+ *     aligned scratch; the general kernel elsewhere (tiny problems), where the geometry has no such form (groups, negative pads, strides above
+ *     8) and where the scratch is too small.
  * MatMulInteger already takes its zero points as device arrays. */
 int chxq_dynamic_quant_params_u8(const float* rmin, const float* rmax, float* scale, uint8_t* zero_point, void* stream);
 int chxq_quantize_linear_dev(const float* x, int64_t n, const float* y_scale, const void* y_zero_point, int32_t y_dtype, int32_t round_mode,

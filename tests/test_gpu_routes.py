@@ -170,3 +170,17 @@ def test_matmul_ragged_k_launches(ops, pkg, orc, dev, batch, M, N, K, launches):
         y = ops.MatMulInteger(at, bt, None if z0 is None else _t(z0, dev), None if z1 is None else _t(z1, dev))
         assert pkg.lib().chxq_launch_count() - before == launches
         assert np.array_equal(y.cpu().numpy(), orc.matmul_integer(a, b, z0, z1)), (z0 is None, z1 is None)
+
+
+# (N, C, H, W, M, k, launches): with a device zero point, one launch of the CUDA-core kernel, or two where the tensor cores are faster
+@pytest.mark.parametrize("N,C,H,W,M,k,launches", [(1, 3, 7, 7, 16, 3, 1), (1, 16, 2, 2, 4, 1, 1), (1, 5, 32, 32, 16, 1, 1), (1, 24, 7, 7, 16, 3, 2), (2, 100, 5, 6, 16, 1, 2),
+                                                  (16, 3, 24, 23, 32, 3, 2)])
+def test_conv_integer_device_zero_point_launches(ops, pkg, orc, dev, N, C, H, W, M, k, launches):
+    rng = np.random.default_rng(C + M)
+    x, w = _rand(rng, (N, C, H, W), np.uint8), _rand(rng, (M, C, k, k), np.uint8)
+    zw = _rand(rng, M, np.uint8)
+    args = (_t(x, dev), _t(w, dev), _t(np.array([77], np.uint8), dev), _t(zw, dev), (1, 1), (k // 2, k // 2))
+    before = pkg.lib().chxq_launch_count()
+    y = ops.ConvInteger(*args)
+    assert pkg.lib().chxq_launch_count() - before == launches
+    assert np.array_equal(y.cpu().numpy(), orc.conv_integer(x, w, 77, zw, (1, 1), (k // 2, k // 2)))
