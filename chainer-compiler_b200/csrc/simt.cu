@@ -387,10 +387,9 @@ __global__ void __launch_bounds__(256) maxpool_u8_nhwc_scalar_kernel(
 }
 
 // y[n, c] = (float(sum_i (x[n,i,c] - zp)) / float(HW)) * scale.  One thread per (n, c); threads of
-// a warp read consecutive channels, so every load instruction is a coalesced row segment.
+// a warp read consecutive channels, so every load instruction is a coalesced row segment.  No early launch of the next kernel (pdl.cuh).
 __global__ void __launch_bounds__(256) global_avgpool_dq_kernel(
         const uint8_t* __restrict__ x, int N, int HW, int C, float scale, int zp, float* __restrict__ y) {
-    pdl_launch_dependents();
     pdl_dependency_wait();
     const int64_t total = (int64_t)N * C;
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -597,10 +596,11 @@ __device__ __forceinline__ void transpose4x4_bytes(uint32_t (&r)[4]) {
     r[3] = __byte_perm(t1, t3, 0x7632);
 }
 
+// (No early launch of the next kernel, see pdl.cuh: [4, 1326, 14, 14] to NHWC, call after call, 15 -> 10 us; the pass behind a convolution of
+// 28 x 28 maps gains with it, 64 -> 62 us for the operator.)
 template <bool kToNhwc>
 __global__ void __launch_bounds__(256) transpose_u8_tile_kernel(const uint8_t* __restrict__ x, int C, int HW, int ld, uint8_t* __restrict__ y) {
     __shared__ uint32_t tw[kTrP][kTrPitchW];
-    pdl_launch_dependents();
     pdl_dependency_wait();
     const int n = blockIdx.z, c0 = blockIdx.y * kTrC, p0 = blockIdx.x * kTrP, tid = threadIdx.x;
     const uint8_t* nchw_in = x + (int64_t)n * C * HW;
@@ -669,63 +669,6 @@ __global__ void __launch_bounds__(256) transpose_u8_tile_kernel(const uint8_t* _
                 *reinterpret_cast<uint32_t*>(dst) = r[i];
             } else {
                 for (int j = 0; j < 4 && pp + j < HW; ++j) dst[j] = (uint8_t)(r[i] >> (8 * j));
-            }
-        }
-    }
-}
-
-// NHWC -> NCHW for maps whose extent is no multiple of four, 128 positions x 64 channels per block: a channel's row then starts wherever
-// c * HW falls, and a warp writes its 128 bytes as the aligned words that cover them, each put together from two words of shared memory,
-// where the form above stores byte by byte.  (Where the form above has whole words it is the faster of the two: 25.7 MB of
-// 28 x 28 maps in 13 us against 27.)
-constexpr int kBackP = 128, kBackPitchW = 33;
-__global__ void __launch_bounds__(256) nhwc_to_nchw_u8_kernel(const uint8_t* __restrict__ x, int C, int HW, int ld, uint8_t* __restrict__ y) {
-    pdl_launch_dependents();
-    pdl_dependency_wait();
-    __shared__ uint32_t tw[64][kBackPitchW];  // [channel][position / 4]: four positions of a channel per word
-    const int n = blockIdx.z, c0 = blockIdx.y * 64, p0 = blockIdx.x * kBackP, tid = threadIdx.x;
-    const uint8_t* in = x + (int64_t)n * HW * ld;
-    const int cq = tid % 16, pq = tid / 16;  // load side: channels 4cq .. +3, positions 4pq .. +3 and 64 further
-    const bool words_ok = (ld % 4 == 0) && ((reinterpret_cast<uintptr_t>(x) & 3u) == 0);
-    const int c = c0 + 4 * cq;
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        uint32_t r[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int p = p0 + 4 * (pq + 16 * h) + j;
-            uint32_t v = 0u;
-            if (p < HW && c < C) {
-                const uint8_t* src = in + (int64_t)p * ld + c;
-                if (words_ok && c + 4 <= ld) {
-                    v = __ldg(reinterpret_cast<const uint32_t*>(src));
-                } else {
-                    for (int k = 0; k < 4 && c + k < C; ++k) v |= (uint32_t)src[k] << (8 * k);
-                }
-            }
-            r[j] = v;
-        }
-        transpose4x4_bytes(r);  // r[i] = the four positions of channel c + i
-#pragma unroll
-        for (int i = 0; i < 4; ++i) tw[4 * cq + i][pq + 16 * h] = r[i];
-    }
-    __syncthreads();
-    const int len = min(kBackP, HW - p0);  // positions of this tile
-    const int lane = tid % 32;
-    for (int k = tid / 32; k < 64 && c0 + k < C; k += 8) {
-        uint8_t* dst = y + ((int64_t)n * C + c0 + k) * HW + p0;
-        const int mis = (int)(reinterpret_cast<uintptr_t>(dst) & 3u);
-        // word i covers the positions 4i - mis .. +3
-        for (int i = lane; 4 * i - mis < len; i += 32) {
-            const uint32_t hi = i < 32 ? tw[k][i] : 0u, lo = i > 0 ? tw[k][i - 1] : 0u;
-            const uint32_t v = mis == 0 ? hi : __funnelshift_r(lo, hi, 32 - 8 * mis);
-            const int first = 4 * i - mis;
-            if (first >= 0 && first + 4 <= len) {
-                *reinterpret_cast<uint32_t*>(dst + first) = v;
-            } else {
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    if (first + j >= 0 && first + j < len) dst[first + j] = (uint8_t)(v >> (8 * j));
             }
         }
     }
@@ -880,11 +823,9 @@ static int transpose_dispatch(const void* x, int elem_bytes, int N, int C, int H
     cudaStream_t s = as_stream(stream);
     if (elem_bytes == 1) {
         // 1-byte maps: the tiled kernel (32-bit words on the NCHW side, 128-bit words on the NHWC side)
-        const bool ragged = !to_nhwc && (HW % 4 != 0 || (reinterpret_cast<uintptr_t>(y) & 3u) != 0);
-        const int tile = ragged ? kBackP : kTrP;
-        dim3 tgrid((HW + tile - 1) / tile, ((to_nhwc ? ld : C) + kTrC - 1) / kTrC, N);
+        dim3 tgrid((HW + kTrP - 1) / kTrP, ((to_nhwc ? ld : C) + kTrC - 1) / kTrC, N);
         CHXQ_CHECK_ARG(tgrid.y <= 65535, "layout transform: too many channels for the grid");
-        CHXQ_CUDA(launch_pdl(to_nhwc ? transpose_u8_tile_kernel<true> : (ragged ? nhwc_to_nchw_u8_kernel : transpose_u8_tile_kernel<false>), tgrid, 256, 0, s,
+        CHXQ_CUDA(launch_pdl(to_nhwc ? transpose_u8_tile_kernel<true> : transpose_u8_tile_kernel<false>, tgrid, 256, 0, s,
                              static_cast<const uint8_t*>(x), C, HW, ld, static_cast<uint8_t*>(y)));
         count_launch(1);
         return CHXQ_OK;
