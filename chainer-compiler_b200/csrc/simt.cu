@@ -431,6 +431,12 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool va
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(gmem), "r"(bytes) : "memory");
 }
 
+__device__ __forceinline__ void cp_async4(void* smem, const void* gmem, bool valid) {
+    const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
+    const int bytes = valid ? 4 : 0;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(gmem), "r"(bytes) : "memory");
+}
+
 // volatile: keeps the load where it stands, ahead of the multiply-adds it overlaps (the compiler sinks a plain load to its first use)
 __device__ __forceinline__ float4 lds128(uint32_t addr) {
     float4 v;
@@ -472,7 +478,11 @@ __global__ void __launch_bounds__(kLinThreads, 1) linear_f32_kernel(
                     const bool ok = row_ok[i] && k < K;
                     cp_async16(dst + kStep * i * T::kPitch, ok ? src[i] + sl * T::KS : x, ok);
                 } else {
-                    for (int e = 0; e < 4; ++e) dst[kStep * i * T::kPitch + e] = row_ok[i] && k + e < K ? src[i][sl * T::KS + e] : 0.f;
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const bool ok = row_ok[i] && k + e < K;
+                        cp_async4(dst + kStep * i * T::kPitch + e, ok ? src[i] + sl * T::KS + e : x, ok);
+                    }
                 }
             }
         }
@@ -552,6 +562,93 @@ cudaError_t launch_linear(const float* x, const float* w, const float* b, int N,
     // finish last ([256, 2048] x [1000, 2048]^T: 78 us instead of 49, call after call).
     linear_f32_kernel<T><<<grid, kLinThreads, T::kSmem, s>>>(x, w, b, N, K, O, y);
     return cudaGetLastError();
+}
+
+// The same chains with 4 x 4 outputs per thread, the next K slice fetched into registers while the current one is consumed and two slices in
+// shared memory: 27 KB per block where the pipelined 4 x 4 tile takes 104 KB, so that several blocks share an SM.  That wins where there are
+// more blocks than two per SM and where a block has little to do (short K); rows of K % 4 != 0 floats it reads with plain loads, where the
+// pipelined kernel needs four copies for sixteen bytes.  One B200, this kernel against the pipelined 4 x 4 tile: [1024, 1000] x [1000, 1000]^T 79
+// and 87 us, [256, 1001] x [4000, 1001]^T 88 and 112, [512, 19] x [1500, 19]^T 6.4 and 14.6, but [256, 2048] x [1000, 2048]^T 60 and 49.5.
+constexpr int kLinKS = 32;     // K slice
+constexpr int kLinPitch = 36;  // floats
+
+__global__ void __launch_bounds__(kLinThreads) linear_f32_regs_kernel(
+        const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ b, int N, int K, int O, float* __restrict__ y) {
+    __shared__ __align__(16) float Xs[2][32][kLinPitch];
+    __shared__ __align__(16) float Ws[2][64][kLinPitch];
+    const int tid = threadIdx.x;
+    const int tn = tid / 16, to = tid % 16;
+    const int n0 = blockIdx.y * 32, o0 = blockIdx.x * 64;
+    const bool vec = (K % 4 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15u) == 0) && ((reinterpret_cast<uintptr_t>(w) & 15u) == 0);
+    // staging assignment: float4 number f = tid + 128 i of a tile covers row f / 8, k offset 4 (f % 8): two of X, four of W
+    const int sr = tid / 8, sk = (tid % 8) * 4;
+    auto fetch = [&](const float* base, int row, int rows, int k0) -> float4 {
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (row < rows) {
+            const float* p = base + (int64_t)row * K + k0 + sk;
+            if (vec && k0 + sk + 4 <= K) {
+                v = *reinterpret_cast<const float4*>(p);
+            } else {
+                if (k0 + sk + 0 < K) v.x = p[0];
+                if (k0 + sk + 1 < K) v.y = p[1];
+                if (k0 + sk + 2 < K) v.z = p[2];
+                if (k0 + sk + 3 < K) v.w = p[3];
+            }
+        }
+        return v;
+    };
+    float acc[4][4] = {};
+    float4 px[2], pw[4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) px[i] = fetch(x, n0 + sr + 16 * i, N, 0);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) pw[i] = fetch(w, o0 + sr + 16 * i, O, 0);
+    int buf = 0;
+    for (int k0 = 0; k0 < K; k0 += kLinKS, buf ^= 1) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) *reinterpret_cast<float4*>(&Xs[buf][sr + 16 * i][sk]) = px[i];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(&Ws[buf][sr + 16 * i][sk]) = pw[i];
+        __syncthreads();
+        if (k0 + kLinKS < K) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) px[i] = fetch(x, n0 + sr + 16 * i, N, k0 + kLinKS);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) pw[i] = fetch(w, o0 + sr + 16 * i, O, k0 + kLinKS);
+        }
+        // Elements past K are zero in both operands; fma(0, 0, acc) leaves acc as it is, so the slice is always run in full.
+#pragma unroll
+        for (int k4 = 0; k4 < kLinKS; k4 += 4) {
+            float4 xv[4], wv[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) xv[i] = *reinterpret_cast<const float4*>(&Xs[buf][tn * 4 + i][k4]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) wv[j] = *reinterpret_cast<const float4*>(&Ws[buf][to + 16 * j][k4]);
+            // k ascending per accumulator; the sixteen accumulators advance together, so that a fused multiply-add never waits
+            // for the one before it (there is only one warp per scheduler to hide that latency)
+            const float xa[4][4] = {{xv[0].x, xv[0].y, xv[0].z, xv[0].w}, {xv[1].x, xv[1].y, xv[1].z, xv[1].w},
+                                    {xv[2].x, xv[2].y, xv[2].z, xv[2].w}, {xv[3].x, xv[3].y, xv[3].z, xv[3].w}};
+            const float wa[4][4] = {{wv[0].x, wv[0].y, wv[0].z, wv[0].w}, {wv[1].x, wv[1].y, wv[1].z, wv[1].w},
+                                    {wv[2].x, wv[2].y, wv[2].z, wv[2].w}, {wv[3].x, wv[3].y, wv[3].z, wv[3].w}};
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) acc[i][j] = __fmaf_rn(xa[i][kk], wa[j][kk], acc[i][j]);
+        }
+        // the buffer written next iteration is the other one; its readers finished before this iteration's barrier
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int n = n0 + tn * 4 + i;
+        if (n >= N) continue;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int o = o0 + to + 16 * j;
+            if (o < O) y[(int64_t)n * O + o] = __fadd_rn(acc[i][j], b ? b[o] : 0.f);
+        }
+    }
 }
 
 // NCHW <-> NHWC transposes through a 32x32 shared tile over the (C, H*W) plane.
@@ -795,17 +892,24 @@ extern "C" int chxq_global_avgpool_dq_nhwc(const uint8_t* x, int32_t N, int32_t 
 
 extern "C" int chxq_linear_f32(const float* x, const float* w, const float* b, int32_t N, int32_t K, int32_t O, float* y, void* stream) {
     CHXQ_CHECK_ARG(x && w && y && N > 0 && K > 0 && O > 0, "Linear: bad arguments");
-    // The largest register tile that still puts a block on every second SM (4 x 4: 2048 outputs per block; measured at K = 2048, O = 1000:
-    // 192 rows 46 us as 4 x 4 and 48 as 2 x 2, 128 rows 44 and 38); for a few tens of rows the single-output tile, whose chains are
-    // the shortest.
+    // The largest register tile that still puts a block on every second SM (4 x 4: 2048 outputs per block), and for few outputs the
+    // single-output tile, whose chains are the shortest, as long as no SM has more than two blocks of it at a time.  Lines from 1338 shapes on
+    // one B200, in us: K = 2048, O = 1000: 192 rows 49.5 as 4 x 4 and 51.7 as 2 x 2, 128 rows 49.4 and 41.2; [16, 512] x [1000, 512]^T 6.4 as 1 x 1
+    // and 8.9 as 2 x 2, [40, 512] 14.6 and 8.9, [24, 66] x [1000, 66]^T 5.6 and 5.3 (K <= 64 is over before slices of 128 pay).  The kernel with
+    // registers takes what the pipelined tiles do not win: more than two 4 x 4 blocks per SM, K < 400 there, rows that are no whole 16-byte
+    // pieces, and from 80,000 outputs on K <= 32 ([40, 32] x [4000, 32]^T 5.2 against 6.4).
     const int64_t outputs = (int64_t)N * O;
+    const bool rows16 = K % 4 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15u) == 0;
     cudaStream_t s = as_stream(stream);
-    if (outputs >= (int64_t)80 * 2048)
-        CHXQ_CUDA((launch_linear<LinTile<4, 4, 8, 64, 4, 2>>(x, w, b, N, K, O, y, s)));
-    else if (outputs >= 40000)
-        CHXQ_CUDA((launch_linear<LinTile<2, 2, 8, 64, 5, 3>>(x, w, b, N, K, O, y, s)));
-    else
+    auto two_per_sm = [&](int o, int n) { return (int64_t)((O + o - 1) / o) * ((N + n - 1) / n) <= 2 * 148; };  // blocks of n x o outputs
+    if (K > 64 && two_per_sm(32, 4))
         CHXQ_CUDA((launch_linear<LinTile<1, 1, 4, 128, 5, 5>>(x, w, b, N, K, O, y, s)));
+    else if (outputs < 80000 || (outputs < 80 * 2048 && rows16 && K > 32))
+        CHXQ_CUDA((launch_linear<LinTile<2, 2, 8, 64, 5, 3>>(x, w, b, N, K, O, y, s)));
+    else if (two_per_sm(64, 32) && rows16 && K >= 400)
+        CHXQ_CUDA((launch_linear<LinTile<4, 4, 8, 64, 4, 2>>(x, w, b, N, K, O, y, s)));
+    else
+        linear_f32_regs_kernel<<<dim3((O + 63) / 64, (N + 31) / 32), kLinThreads, 0, s>>>(x, w, b, N, K, O, y);
     CHXQ_LAUNCH_CHECK();
     return CHXQ_OK;
 }

@@ -202,3 +202,16 @@ def test_linear_tiles(ops, orc, dev, n, k, o):
     x, w = rng.standard_normal((n, k)).astype(np.float32), rng.standard_normal((o, k)).astype(np.float32)
     b = rng.standard_normal(o).astype(np.float32)
     assert np.array_equal(ops.Linear(_t(x, dev), _t(w, dev), _t(b, dev)).cpu().numpy(), orc.linear_f32(x, w, b))
+
+
+@pytest.mark.parametrize("n,k,o", [(36, 65, 1000), (37, 65, 1000), (39, 64, 1000), (80, 33, 1000), (90, 30, 1000), (90, 36, 1000), (80, 399, 1003), (164, 399, 1000), (164, 400, 1003), (606, 404, 1001),
+                                   (33, 5, 65)])
+def test_linear_routes(ops, orc, dev, n, k, o):
+    """Both sides of each line between the Linear kernels, with rows on 16-byte boundaries and off them."""
+    rng = np.random.default_rng(n + k + o)
+    x, w = rng.standard_normal((n, k)).astype(np.float32), rng.standard_normal((o, k)).astype(np.float32)
+    want = orc.linear_f32(x, w, np.zeros(o, np.float32))
+    odd = torch.zeros(n * k + 1, device=dev)
+    odd[1:] = _t(x, dev).reshape(-1)
+    for xt in (_t(x, dev), odd[1:].reshape(n, k)):
+        assert np.array_equal(ops.Linear(xt, _t(w, dev)).cpu().numpy(), want)
