@@ -2,6 +2,7 @@
 // argument validation, convolution geometry, path selection, workspace carving, and the small
 // pre-pass kernels that feed the tensor-core kernel (operand repacking and zero-point terms).
 #include <cooperative_groups.h>
+#include <math.h>
 #include <string.h>
 
 #include <atomic>
@@ -745,16 +746,23 @@ bool gemm_tc_eligible(const void* a, int64_t M, int64_t N, int64_t K) {
 }
 
 // Rows of A that do not start on sixteen-byte boundaries (K % 16 != 0) can reach the tensor cores through a copy at a wider pitch, in two
-// launches per matrix; the CUDA-core kernel takes the whole batch in one.  Which of them is estimated to finish first: the copy and the
-// product cost 7 us a matrix and a pass over both operands, the CUDA-core kernel 2 us, 27 steps of its K chain a microsecond and 7.3 million
-// multiply-adds a microsecond.  One B200, device time, copy / CUDA cores: 512 x [49 x 49 x 50] 3600 / 23 us, 8 x [512 x 512 x 500] 67 / 147 us,
-// 49 x 49 x 50 7.0 / 4.1 us, 128 x 128 x 250 7.0 / 12.4 us, 509 x 3073 x 1283 22 / 293 us; over 220 products of 1 to 64 matrices, extents up
-// to 3000, the choice costs 0.2 % on the geometric mean against the faster of the two (the copy alone 152 %, the CUDA cores alone 34 %).
-bool gemm_tc_via_copy(int64_t batch, int64_t M, int64_t N, int64_t K) {
+// launches per matrix; the CUDA-core kernel takes the whole batch in one.  Which of them is estimated to finish first.  The copy and the
+// product cost 6.2 us a matrix, a pass over both operands, a chain of K blocks, 4 us for zero points of a by k, 1 us to requantize and, with
+// the general epilogue (int8 outputs, round half to even, a zero point of b), 2 us more and up to 24 per wave of its 128-column tiles.  The
+// CUDA-core kernel costs 2 us and, partly at the same time, its K chain at 27 steps a microsecond and its multiply-adds at 7.3 million a
+// microsecond.  One B200, device time, copy / CUDA cores: 512 x [49 x 49 x 50] 3600 / 23 us, 8 x [512 x 512 x 500] 67 / 147 us,
+// 49 x 49 x 50 7.0 / 4.1 us, 128 x 128 x 250 7.0 / 12.4 us, 509 x 3073 x 1283 22 / 293 us, requantized to int8 280 x 171 x 44 36 / 6.3 us and
+// 996 x 1995 x 447 44 / 130 us.  Over 220 products of 1 to 64 matrices, extents up to 3000, the choice costs 0.04 % on the geometric mean
+// against the faster of the two (the copy alone 152 %, the CUDA cores alone 34 %); over 200 requantized ones 0.8 % (66 %, 22 %).
+bool gemm_tc_via_copy(int64_t batch, int64_t M, int64_t N, int64_t K, bool za_vector, bool requant, bool general_epilogue) {
     if (K % 16 == 0 || K < 16 || M < 1 || N < 1 || M >= (1ll << 31) || N >= (1ll << 31) || K >= (1ll << 20)) return false;
-    const double copy_us = (double)batch * (7.0 + ((double)M + (double)N) * (double)K / 6e5);
-    const double simt_us = 2.0 + (double)K / 27.0 + (double)batch * (double)M * (double)N * (double)K / 7.3e6;
-    return copy_us < simt_us;
+    double copy_us = 6.2 + ((double)M + (double)N) * (double)K / 6e5 + (double)K / 1200.0 + (za_vector ? 4.0 : 0.0) + (requant ? 1.0 : 0.0);
+    if (general_epilogue) {
+        const int64_t tiles = ((M + 127) / 128) * ((N + 127) / 128), waves = (tiles + 147) / 148;
+        copy_us += 2.0 + 24.0 * (double)waves * (N < 128 ? (double)N / 128.0 : 1.0);
+    }
+    const double chain_us = (double)K / 27.0, macs_us = (double)batch * (double)M * (double)N * (double)K / 7.3e6;
+    return (double)batch * copy_us < 2.0 + sqrt(chain_us * chain_us + macs_us * macs_us);
 }
 
 int gemm_dispatch(
@@ -763,7 +771,8 @@ int gemm_dispatch(
         cudaStream_t s) {
     if (batch == 0 || M == 0 || N == 0) return CHXQ_OK;
     const bool tc_ok = gemm_tc_eligible(a, M, N, K) && ((M * K) % 16 == 0 || batch == 1);
-    bool use_tc = path == CHXQ_PATH_TENSOR || (path == CHXQ_PATH_AUTO && (tc_ok || gemm_tc_via_copy(batch, M, N, K)));
+    const bool general_epilogue = epi.mode == kEpiRequant && (epi.rq.y_signed || epi.rq.round_mode != 0 || zb.len > 0);
+    bool use_tc = path == CHXQ_PATH_TENSOR || (path == CHXQ_PATH_AUTO && (tc_ok || gemm_tc_via_copy(batch, M, N, K, za.len > 1, epi.mode == kEpiRequant, general_epilogue)));
     if (path == CHXQ_PATH_TENSOR && !tc_ok)
         return set_error(CHXQ_ERR_UNSUPPORTED, "%s: tensor-core path needs K %% 16 == 0 and a 16-byte aligned A (M=%lld N=%lld K=%lld)", op,
                          (long long)M, (long long)N, (long long)K);

@@ -157,7 +157,7 @@ def test_conv_pixel_sums_fit_the_reported_workspace(ops, dev, N, C, H, W, M, k, 
 
 
 # (batch, M, N, K, launches): the copy and the product (two launches a matrix) where they are faster than the one of the CUDA cores
-@pytest.mark.parametrize("batch,M,N,K,launches", [(1, 1, 1, 137, 2), (1, 7, 3, 145, 2), (1, 8, 63, 201, 2), (1, 9, 65, 255, 2), (1, 129, 64, 193, 2), (2, 5, 21, 401, 4),
+@pytest.mark.parametrize("batch,M,N,K,launches", [(1, 1, 1, 249, 2), (1, 7, 3, 259, 2), (1, 8, 63, 265, 2), (1, 9, 65, 255, 2), (1, 129, 64, 321, 2), (2, 5, 21, 561, 4),
                                                   (3, 130, 257, 1283, 6), (1, 49, 49, 50, 1), (512, 49, 49, 50, 1), (5, 70, 33, 197, 1)])
 def test_matmul_ragged_k_launches(ops, pkg, orc, dev, batch, M, N, K, launches):
     rng = np.random.default_rng(batch + M + N + K)
@@ -184,3 +184,18 @@ def test_conv_integer_device_zero_point_launches(ops, pkg, orc, dev, N, C, H, W,
     y = ops.ConvInteger(*args)
     assert pkg.lib().chxq_launch_count() - before == launches
     assert np.array_equal(y.cpu().numpy(), orc.conv_integer(x, w, 77, zw, (1, 1), (k // 2, k // 2)))
+
+
+# requantized products of ragged K: the general epilogue (int8 outputs here) moves the line
+@pytest.mark.parametrize("M,N,K,launches_u8,launches_s8", [(64, 208, 188, 2, 1), (280, 171, 44, 1, 1), (996, 901, 447, 2, 2), (2, 4, 725, 2, 2)])
+def test_qlinear_matmul_ragged_k_launches(ops, pkg, orc, dev, M, N, K, launches_u8, launches_s8):
+    rng = np.random.default_rng(M + K)
+    a, b = _rand(rng, (M, K), np.uint8), _rand(rng, (K, N), np.int8)
+    ys = float(0.02 * 0.0015 * 74 * 73 * np.sqrt(K) / 40)
+    acc = orc.matmul_integer(a, b, np.array([9], np.uint8), None)
+    for oz, launches in ((np.uint8(11), launches_u8), (np.int8(-5), launches_s8)):
+        before = pkg.lib().chxq_launch_count()
+        y = ops.QLinearMatMul(_t(a, dev), 0.02, np.uint8(9), _t(b, dev), 0.0015, np.int8(0), ys, oz)
+        assert pkg.lib().chxq_launch_count() - before == launches
+        want = orc.requantize(acc, 1.0, np.array([np.float32(0.02) * np.float32(0.0015)], np.float32), ys, int(oz), y_dtype=type(oz))
+        assert np.array_equal(y.cpu().numpy(), want)
