@@ -259,12 +259,15 @@ int launch_tc_igemm(const TcProblem& q, cudaStream_t s) {
     if (q.group_cols > 0 && q.group_cols % 64 != 0)
         return set_error(CHXQ_ERR_UNSUPPORTED, "tensor-core kernel: grouped convolution needs a multiple of 64 output channels per group");
     // Few tiles, many K blocks: clusters that share a tile's K blocks (see tc_igemm_kernel).  At least two blocks per CTA, and all clusters
-    // resident at once.  One B200: ResNet-50 batch 1 op by op 453 -> 351 us, the MLP of 64
-    // rows 66 -> 51 us (with programmatic dependent launch of this kernel, same step).
+    // resident at once: 33 of four, not 148 / 4, because a cluster stays inside a group of SMs ([8, 1232] x [1232, 64 n]: 33 tiles 12.2 us, 34 to 37
+    // tiles as clusters of four 16.7 us, as pairs 12.2 us).  The general epilogue stays one CTA per tile: it is built for 128-column tiles only.
+    // One B200: ResNet-50 batch 1 op by op 453 -> 351 us, the MLP of 64 rows 66 -> 51 us (with programmatic dependent launch of this
+    // kernel, same step).
     const int64_t num_kb = (int64_t)q.KH * q.KW * (q.c_pad / q.bk), tiles64 = pos_tiles * ((q.cols + 63) / 64);
     int split = 1;
     if (chxq::g_variant.load(std::memory_order_relaxed) == 0 && epi_kind != tc::kEpiKGeneric && q.bk >= 64 && q.pool_ho == 0)
-        split = tiles64 * 4 <= num_sms() && num_kb >= 8 ? 4 : (tiles64 * 2 <= num_sms() && num_kb >= 4 ? 2 : 1);
+        split = num_kb >= 8 && tiles64 * 4 <= num_sms() && tiles64 <= tc::split_slots(4) ? 4 :
+                (num_kb >= 4 && tiles64 * 2 <= num_sms() && tiles64 <= tc::split_slots(2) ? 2 : 1);
     const int bn = q.group_cols > 0 || split > 1 ? 64 : (epi_kind == tc::kEpiKGeneric ? 128 : (q.bn ? q.bn : pick_bn(q.cols, pos_tiles)));
     p.col_tiles = (q.cols + bn - 1) / bn;
     const int64_t total_tiles = pos_tiles * p.col_tiles;

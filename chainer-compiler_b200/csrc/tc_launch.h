@@ -83,6 +83,7 @@ constexpr int kEpiKU8Fold = 3;   // uint8 with one folded multiplier per channel
 int launch_tc_bk32(int bn, int epi, int split, const CUtensorMap& tmA, const CUtensorMap& tmB, const TcParams& p, int grid, cudaStream_t s);
 int launch_tc_bk64(int bn, int epi, int split, const CUtensorMap& tmA, const CUtensorMap& tmB, const TcParams& p, int grid, cudaStream_t s);
 int launch_tc_bk128(int bn, int epi, int split, const CUtensorMap& tmA, const CUtensorMap& tmB, const TcParams& p, int grid, cudaStream_t s);
+int split_slots(int split);  // clusters of 2 or 4 CTAs of that kernel that are resident at once
 // Grouped-tile kernel (tc_kernel2.cuh); bn is 64 or 128, epi is kEpiKU8 or kEpiKU8Fold.
 // pool: the fused max-pooling form (bn 64, no residual; 64-byte K tiles only), with or without halo tiles.
 int launch_tc2_bk64_pool(int epi, bool halo, const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmY, const CUtensorMap& tmR, const TcParams& p,

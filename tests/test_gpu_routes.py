@@ -199,3 +199,14 @@ def test_qlinear_matmul_ragged_k_launches(ops, pkg, orc, dev, M, N, K, launches_
         assert pkg.lib().chxq_launch_count() - before == launches
         want = orc.requantize(acc, 1.0, np.array([np.float32(0.02) * np.float32(0.0015)], np.float32), ys, int(oz), y_dtype=type(oz))
         assert np.array_equal(y.cpu().numpy(), want)
+
+
+# as many clusters of four CTAs as are resident at once, one more (pairs then), and around the last pair
+@pytest.mark.parametrize("tiles", [33, 34, 37, 74, 75])
+def test_split_k_last_cluster(ops, dev, tiles):
+    """|sum| < 2^24: the fp64 product is exact."""
+    M, N, K = 8, 64 * tiles - 3, 1232
+    gen = torch.Generator(device=dev).manual_seed(tiles)
+    a = torch.randint(0, 256, (M, K), dtype=torch.uint8, device=dev, generator=gen)
+    b = torch.randint(-127, 128, (K, N), dtype=torch.int8, device=dev, generator=gen)
+    assert torch.equal(ops.MatMulInteger(a, b, None, None), (a.double() @ b.double()).to(torch.int32))
