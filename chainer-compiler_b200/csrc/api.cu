@@ -1589,7 +1589,8 @@ static bool conv_dev_tc_pays(const chxq_conv_geom& g, bool w_zp) {
 
 extern "C" size_t chxq_conv_dev_workspace(const chxq_conv_geom* g) {
     if (!g || validate_geom("conv workspace", g) != CHXQ_OK) return 0;
-    return prep_workspace(*g);
+    PrepPlan P;  // always with a border where the convolution pads: the zero point is not known here
+    return prep_plan(*g, 4, true, true, &P) ? P.total : 0;
 }
 
 extern "C" int chxq_conv_integer_dev_ws(
