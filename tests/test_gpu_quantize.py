@@ -215,3 +215,23 @@ def test_linear_routes(ops, orc, dev, n, k, o):
     odd[1:] = _t(x, dev).reshape(-1)
     for xt in (_t(x, dev), odd[1:].reshape(n, k)):
         assert np.array_equal(ops.Linear(xt, _t(w, dev)).cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 7, 1023, 4 * 256 * 4, (1 << 20) + 2, 8 * 148 * 256 * 16 + 4, 20_000_003])
+def test_minmax_values_and_lengths(ops, dev, n):
+    """The extremes at the first, the last and a middle element; infinities; NaNs, which the reduction passes over.  Lengths with and without a tail
+    behind the last 16 bytes, a last stride that only some threads have, and less than one stride."""
+    gen = torch.Generator(device=dev).manual_seed(n)
+    base = torch.randn(n, device=dev, generator=gen)
+    for lo, hi in ((0, n - 1), (n - 1, 0), (n // 2, n // 3)):
+        for big in (1e3, float("inf")):
+            for nan in (False, True):
+                x = base.clone()
+                if nan and n > 3:
+                    x[torch.randint(0, n, (max(1, n // 5),), device=dev, generator=gen)] = float("nan")
+                x[hi] = big
+                x[lo] = -big
+                v = x[~torch.isnan(x)]
+                assert torch.equal(ops.MinMax(x), torch.stack([v.min(), v.max()])), (lo, hi, big, nan)
+                if n > 1:  # not on a 16-byte boundary
+                    assert torch.equal(ops.MinMax(x[1:]), torch.stack([x[1:][~torch.isnan(x[1:])].min(), x[1:][~torch.isnan(x[1:])].max()]))
