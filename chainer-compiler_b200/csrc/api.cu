@@ -59,6 +59,8 @@ __device__ __forceinline__ uint32_t load4_unaligned(const uint8_t* p, int64_t n)
 // launch in front and global atomics.  A tile: 32-bit loads along N at any alignment of the rows, a 4 x 4 byte transpose in registers, the
 // tile through shared memory as words at an odd pitch, 128-bit stores along K.
 // 8192 x 8192 on one B200: 53 -> 41.5 us against the 64-row form with one byte multiplied at a time (134 MB: 3.2 TB/s).
+// Eight blocks are the largest portable cluster.  Its cost: with K <= 1024 every block has one tile and nothing to fetch ahead, and with K <= 128
+// seven of the eight only take part in the sums.
 constexpr int kTrSplit = 8, kTrRows = 128;
 __device__ __forceinline__ void transpose_b_terms(
         int64_t col_block, int split, const uint8_t* __restrict__ b, int64_t K, int64_t N, int64_t k_pad, uint8_t* __restrict__ bt, const ZpSpec& za,
@@ -1099,7 +1101,10 @@ bool prep_plan(const chxq_conv_geom& g, int y_elem, bool border, bool pixel_sums
     a.c_pitch = P.pl.c_pitch; a.k_total = P.pl.k_total;
     a.pos_tiles = copy ? (int)((Hp * Wp + kPrepPos - 1) / kPrepPos) : 0;
     // Channel tiles side by side where nothing is summed over them; with pixel sums a block keeps its channels, in up to four shares
-    // (each is another load per tap in the epilogue) where the positions alone leave SMs idle.
+    // (each is another load per tap in the epilogue) where the positions alone are fewer than four blocks on each of 148 SMs.  A constant, not
+    // the device's SM count: the workspace size comes from here too, also without a device.  ConvInteger 3 x 3 to 64 channels on one B200, shares /
+    // one share: [1, 512, 14, 14] 17.4 / 26.3 us, [16, 256, 28, 28] 21.6 / 30.0, [32, 256, 28, 28] 30.3 / 38.3; [8, 256, 28, 28] 21.3 / 19.9 and
+    // [64, 128, 28, 28] 32.5 / 29.8 lose a little.
     const int c_tiles = (a.cs + 63) / 64;
     int parts = c_tiles;
     if (pixel_sums) {

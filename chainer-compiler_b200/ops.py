@@ -10,8 +10,8 @@ fallback: without a CUDA device or without the built libraries every op raises.
 
 Array arguments are ``torch`` CUDA tensors, logically NCHW / row-major as in the reference.
 Activation maps that are ``channels_last`` in memory take the NHWC kernels (tensor cores,
-depthwise kernel) and yield ``channels_last`` outputs; plain contiguous NCHW maps take the general
-CUDA-core kernels.  ``Scalar`` arguments are Python / numpy scalars; a zero point carries its dtype
+depthwise kernel) as they are and yield ``channels_last`` outputs; plain contiguous NCHW maps yield NCHW outputs
+(dense convolutions run on the tensor cores all the same, behind a pass that rewrites the map).  ``Scalar`` arguments are Python / numpy scalars; a zero point carries its dtype
 as a numpy scalar (``np.uint8(3)``, ``np.int8(-1)``) the way ``StrictScalar`` does in the reference
 (``runtime/strict_scalar.h:8-34``).
 """
